@@ -233,7 +233,7 @@ void launch_p2r(cgd_handle *h, const double *U, const double *Pr, const double *
   int nIF;
   const GP gp = ranged_gp(h, nIF);
   if (nIF <= 0) return;
-  dim3 grid((h->nz + CF::LC - 1) / CF::LC, nIF);
+  dim3 grid(p2_items<CF>(h->nz), nIF);   // the items of one element run back to back
   k_phase2<N, NT, R><<<grid, CF::THREADS, CF::SMEM, h->stream>>>(gp, U, Pr, T1, C);
 }
 
@@ -1989,8 +1989,8 @@ int cgd_kernel_times(cgd_handle *h, char *names, int32_t names_len, double *ms, 
 // launches over flat work lists.
 // ===========================================================================
 // Work lists of an ensemble: 0 phase-1 tiles of 256/N^2 levels, 1 column-level
-// blocks of 256 (pressure, gather), 2 phase-2 chunks, 3 column blocks, 4 phase-2
-// chunks of the 16-warp form, 5 phase-1 tiles of the split form (HV1Tile: 16
+// blocks of 256 (pressure, gather), 2 phase-2 items, 3 column blocks, 4 phase-2
+// items of the fused form and of the 8-level split form, 5 phase-1 tiles of the split form (HV1Tile: 16
 // levels at p = 4 in FP64, else as list 0)
 constexpr int BATCH_LISTS = 6;
 
@@ -2003,13 +2003,13 @@ struct cgd_batch {
   cudaEvent_t order_ev = nullptr;   // orders a step after the first member's caller stream
   // work lists, one set per candidate order; a candidate is (order, form):
   // candidate c runs order c % NORD in form c / NORD: split into 15 launches
-  // (FORM_SPLIT), split with phase 2 in 16-level CTAs (FORM_SPLIT16, p = 4),
+  // (FORM_SPLIT), split with phase 2 in 8-level CTAs (FORM_SPLIT8, p = 4),
   // as three fused stage launches (FORM_FUSED), or every member's own
   // single-member step on its own stream inside the graph (FORM_MEMBERS;
   // orders 0 and 1: one member after the other, as given or the largest
   // first; order 2: all members as concurrent branches)
   static constexpr int NORD = 3;
-  static constexpr int FORM_SPLIT = 0, FORM_SPLIT16 = 1, FORM_FUSED = 2, FORM_MEMBERS = 3, NFORM = 4;
+  static constexpr int FORM_SPLIT = 0, FORM_SPLIT8 = 1, FORM_FUSED = 2, FORM_MEMBERS = 3, NFORM = 4;
   static constexpr int NCAND = NFORM * NORD;
   WItem *w[NORD][BATCH_LISTS] = {};
   int n[BATCH_LISTS] = {};
@@ -2040,7 +2040,7 @@ struct cgd_batch {
 namespace {
 
 const char *const ORDER_NAME[cgd_batch::NORD] = {"member-major", "largest-member-first", "members-interleaved"};
-const char *const FORM_NAME[cgd_batch::NFORM] = {"split", "split16", "fused", "members"};
+const char *const FORM_NAME[cgd_batch::NFORM] = {"split", "split8", "fused", "members"};
 int form_of(int cand) { return cand / cgd_batch::NORD; }
 // the order's name; in the members form order 2 forks the members at once
 const char *order_name(int cand)
@@ -2052,7 +2052,7 @@ const char *order_name(int cand)
 // levels per phase-2 CTA of a form
 int phase2_levels(int N, int form)
 {
-  if (form == cgd_batch::FORM_SPLIT16) return P2Cfg<5, 0, double, P2_ALT_WARPS>::LC;
+  if (form == cgd_batch::FORM_FUSED || form == cgd_batch::FORM_SPLIT8) return FUSED_P2_LEVELS;
   switch (N) {
     case 2: return P2Cfg<2, 0, double>::LC;
     case 3: return P2Cfg<3, 0, double>::LC;
@@ -2086,13 +2086,7 @@ void batch_lists(const cgd_batch *b, int order, std::vector<WItem> out[BATCH_LIS
   const int DoF = b->N * b->N;
   const int LT = 256 / DoF;
   const int LTW = b->mix ? LT : (b->N == 5 ? HV1Tile<5, double>::LT : LT);   // list 5
-  int LC = 0, LCA = 0;   // phase-2 levels per CTA: default, alternative (p = 4 only)
-  switch (b->N) {
-    case 2: LC = LCA = P2Cfg<2, 0, double>::LC; break;
-    case 3: LC = LCA = P2Cfg<3, 0, double>::LC; break;
-    case 4: LC = LCA = P2Cfg<4, 0, double>::LC; break;
-    default: LC = P2Cfg<5, 0, double>::LC; LCA = P2Cfg<5, 0, double, P2_ALT_WARPS>::LC; break;
-  }
+  const int LC = phase2_levels(b->N, cgd_batch::FORM_SPLIT), LCF = FUSED_P2_LEVELS;
   for (int m = 0; m < nm; ++m) {
     const cgd_handle *h = b->mem[m];
     for (int IF = 0; IF < h->NF; ++IF)
@@ -2100,10 +2094,10 @@ void batch_lists(const cgd_batch *b, int order, std::vector<WItem> out[BATCH_LIS
     const long long ncl = (long long)h->nz * h->NumG;
     for (long long t = 0; t < (ncl + 255) / 256; ++t) per[1][m].push_back({m, (int)t, 0});
     for (int IF = 0; IF < h->NF; ++IF)
-      for (int c = 0; c < (h->nz + LC - 1) / LC; ++c) per[2][m].push_back({m, c, IF});
+      for (int c = 0; c < 2 * ((h->nz + LC - 1) / LC); ++c) per[2][m].push_back({m, c, IF});
     for (int c = 0; c < (h->NumG + COL_WARPS - 1) / COL_WARPS; ++c) per[3][m].push_back({m, c, 0});
     for (int IF = 0; IF < h->NF; ++IF)
-      for (int c = 0; c < (h->nz + LCA - 1) / LCA; ++c) per[4][m].push_back({m, c, IF});
+      for (int c = 0; c < 2 * ((h->nz + LCF - 1) / LCF); ++c) per[4][m].push_back({m, c, IF});
     for (int IF = 0; IF < h->NF; ++IF)
       for (int t = 0; t < (h->nz + LTW - 1) / LTW; ++t) per[5][m].push_back({m, t, IF});
   }
@@ -2131,7 +2125,7 @@ template <int N, int NT, typename R>
 void batch_enqueue_t(cgd_batch *b, WItem *const *w, bool p2alt)
 {
   using CF = P2Cfg<N, NT, R>;
-  using CFA = P2Cfg<N, NT, R, P2_ALT_WARPS>;
+  using CFA = P2Cfg<N, NT, R, P2_ALT_LEVELS>;
   static std::atomic<unsigned long long> attr{0};
   const size_t csmem = (size_t)COL_WARPS * COL_ARR * b->nzmax * sizeof(double);
   if (first_on_device(attr)) {
@@ -2139,7 +2133,7 @@ void batch_enqueue_t(cgd_batch *b, WItem *const *w, bool p2alt)
     cudaFuncSetAttribute(kb_hypervisc1w<N, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)HV1Smem<N, NT, R, HV1Tile<N, R>::LT>::BYTES);
     if constexpr (N == 5)
-      cudaFuncSetAttribute(kb_phase2<N, NT, R, P2_ALT_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(kb_phase2<N, NT, R, P2_ALT_LEVELS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)CFA::SMEM);
     constexpr bool C32 = sizeof(R) == sizeof(float);
     for (auto f : {kb_column<0, C32>, kb_column<1, C32>, kb_column<2, C32>})
@@ -2151,7 +2145,7 @@ void batch_enqueue_t(cgd_batch *b, WItem *const *w, bool p2alt)
     kb_hypervisc1w<N, NT, R><<<b->n[5], HT::THREADS, HV1Smem<N, NT, R, HT::LT>::BYTES, b->stream>>>(w[5], stage);
     kb_gather<sizeof(R) == sizeof(float)><<<b->n[1], 256, 0, b->stream>>>(w[1]);
     if constexpr (N == 5) {
-      if (p2alt) kb_phase2<N, NT, R, P2_ALT_WARPS><<<b->n[4], CFA::THREADS, CFA::SMEM, b->stream>>>(w[4], stage);
+      if (p2alt) kb_phase2<N, NT, R, P2_ALT_LEVELS><<<b->n[4], CFA::THREADS, CFA::SMEM, b->stream>>>(w[4], stage);
       else kb_phase2<N, NT, R><<<b->n[2], CF::THREADS, CF::SMEM, b->stream>>>(w[2], stage);
     } else {
       kb_phase2<N, NT, R><<<b->n[2], CF::THREADS, CF::SMEM, b->stream>>>(w[2], stage);
@@ -2235,7 +2229,7 @@ cudaError_t batch_enqueue_fused_r(cgd_batch *b, WItem *const *w)
 template <int NT, typename R>
 cudaError_t fused_setup_t(cgd_batch *b)
 {
-  using CF = P2Cfg<5, NT, R, FUSED_P2_WARPS>;
+  using CF = P2Cfg<5, NT, R, FUSED_P2_LEVELS>;
   const size_t csm = (size_t)COL_WARPS * COL_ARR * b->nzmax * sizeof(double);
   b->fsmem = std::max(std::max(CF::SMEM, csm), HV1Smem<5, NT, R>::BYTES);
   cudaError_t e = cudaFuncSetAttribute(kb_stage<5, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->fsmem);
@@ -2298,8 +2292,8 @@ cudaError_t batch_enqueue(cgd_batch *b, int cand)
   const int form = form_of(cand);
   if (form == cgd_batch::FORM_FUSED)
     return b->mix ? batch_enqueue_fused_r<float>(b, w) : batch_enqueue_fused_r<double>(b, w);
-  if (b->mix) batch_enqueue_r<float>(b, w, form == cgd_batch::FORM_SPLIT16);
-  else batch_enqueue_r<double>(b, w, form == cgd_batch::FORM_SPLIT16);
+  if (b->mix) batch_enqueue_r<float>(b, w, form == cgd_batch::FORM_SPLIT8);
+  else batch_enqueue_r<double>(b, w, form == cgd_batch::FORM_SPLIT8);
   return cudaSuccess;
 }
 
@@ -2374,7 +2368,7 @@ int cgd_batch_create(cgd_handle *const *members, int32_t nmembers, int32_t flags
                                  : want_members ? cgd_batch::FORM_MEMBERS * cgd_batch::NORD : 0;
     for (int c = 0; c < cgd_batch::NCAND; ++c) {
       const int form = form_of(c);
-      const bool avail = form == cgd_batch::FORM_SPLIT || (form == cgd_batch::FORM_SPLIT16 && b->N == 5) ||
+      const bool avail = form == cgd_batch::FORM_SPLIT || (form == cgd_batch::FORM_SPLIT8 && b->N == 5) ||
                          (form == cgd_batch::FORM_FUSED && fused_ok) ||
                          form == cgd_batch::FORM_MEMBERS;
       b->use[c] = b->autotune ? avail : c == first;

@@ -176,8 +176,11 @@ __device__ __forceinline__ void recu4(double cLL, double cL, double cR, double c
 template <int N, int NT, typename R, int LT_ = 256 / (N * N)>
 struct HV1Smem {
   static constexpr int DoF = N * N, LT = LT_;
+  // row stride of a plane, odd: the levels of a half warp, a row apart, fall
+  // into different banks (with the 16 of p = 3 they all shared one)
+  static constexpr int RS = DoF | 1;
   static constexpr int PLANES = 9 + 3 * NT;
-  static constexpr size_t BYTES = (size_t)PLANES * LT * DoF * sizeof(R);
+  static constexpr size_t BYTES = (size_t)PLANES * LT * RS * sizeof(R);
 };
 
 // Level tile of k_hypervisc1.  At p = 4 in FP64, 16 levels (400 threads,
@@ -193,29 +196,22 @@ struct HV1Tile {
   static constexpr int THREADS = WIDE ? LT * N * N : 256;
   static constexpr int MINB = WIDE ? 3 : 4;
 };
-template <int N, int NT, typename R>
-__device__ __forceinline__ R *hv1_static_smem()
-{
-  using S = HV1Smem<N, NT, R>;
-  __shared__ R s[S::PLANES * S::LT * S::DoF];
-  return s;
-}
 
-// sbuf: the shared arrays (hv1_static_smem, or a kernel's dynamic buffer)
+// sbuf: the shared arrays (a kernel's dynamic buffer)
 template <int N, int NT, typename R, int LT = 256 / (N * N)>
 __device__ __forceinline__ void hypervisc1_body(const GP &P, const double *__restrict__ U, double *__restrict__ C,
                                                 const int tile, const int IF, R *sbuf)
 {
   constexpr bool MIX = sizeof(R) == sizeof(float);
-  constexpr int DoF = N * N;
-  R(*s)[LT * DoF] = reinterpret_cast<R(*)[LT * DoF]>(sbuf);
+  constexpr int DoF = N * N, RS = HV1Smem<N, NT, R, LT>::RS;
+  R(*s)[LT * RS] = reinterpret_cast<R(*)[LT * RS]>(sbuf);
   const int t = threadIdx.x;
   const int lvl = t % LT, ID = t / LT;
   const int I = ID % N, Jn = ID / N;
   const int l = tile * LT + lvl;
   const int nz = P.nz, NumG = P.NumG;
   const bool act = (ID < DoF) && (l < nz);
-  const int si = lvl * DoF + ID, row = lvl * DoF;
+  const int si = lvl * RS + ID, row = lvl * RS;
   const size_t cs = (size_t)DoF * nz;
   int g = 0;
   R d11 = 0, d12 = 0, d21 = 0, d22 = 0;

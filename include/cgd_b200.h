@@ -402,8 +402,8 @@ int cgd_batch_step(cgd_batch *b, double *const *U, const double *dt, int32_t nst
  * context usable.  Runs on the current device and synchronises it.  No
  * counterpart in the reference. */
 int cgd_grid_barrier_check(int32_t rounds, int32_t absent, double limit_s, int32_t *violations);
-/* The chosen candidate and the timed ones ("order=...;stage=split|fused;
- * phase2_levels=<levels per phase-2 CTA>;<order>/<split|split8|fused>=..ms;..."). */
+/* The chosen candidate and the timed ones ("order=...;stage=split|fused|members;
+ * phase2_levels=<levels per phase-2 CTA>;<order>/<split|split8|fused|members>=..ms;..."). */
 int cgd_batch_tuning(cgd_batch *b, char *desc, int32_t len);
 int cgd_batch_get_stream(cgd_batch *b, void **stream);
 void cgd_batch_destroy(cgd_batch *b);
