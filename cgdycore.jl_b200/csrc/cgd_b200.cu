@@ -327,6 +327,28 @@ void column(cgd_handle *h, const ColArgs &a)
   else column_t<MODE, false>(h, a);
 }
 
+template <int N>
+int launch_cells_n(cgd_handle *h, const CellArgs &a, int OP, double *cell)
+{
+  using CF = CellCfg<N>;
+  static std::atomic<unsigned long long> attr{0};
+  if (first_on_device(attr))
+    CK(cudaFuncSetAttribute(k_cells<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::smem(CELL_MAX)));
+  const dim3 grid((h->nz + CF::LT - 1) / CF::LT, h->NF);
+  k_cells<N><<<grid, 256, CF::smem(a.n), h->stream>>>(h->gp, a, h->ointer, OP, cell);
+  return CGD_OK;
+}
+
+int launch_cells(cgd_handle *h, const CellArgs &a, int OP, double *cell)
+{
+  switch (h->N) {
+    case 2: return launch_cells_n<2>(h, a, OP, cell);
+    case 3: return launch_cells_n<3>(h, a, OP, cell);
+    case 4: return launch_cells_n<4>(h, a, OP, cell);
+    default: return launch_cells_n<5>(h, a, OP, cell);
+  }
+}
+
 // Event between two kernels of a step launched without the graph (the
 // profiled step, see cgd_ros_step).
 void rec(cgd_handle *h, int i)
@@ -1514,20 +1536,6 @@ int out_cells(cgd_handle *h, double *cell, size_t count, double **dev)
 
 size_t out_count(const cgd_handle *h, int OP) { return (size_t)OP * OP * h->nz * h->NF; }
 
-unsigned out_blocks(const cgd_handle *h, int OP) { return (unsigned)((out_count(h, OP) + 255) / 256); }
-
-void launch_vort(cgd_handle *h, const double *U, int OP, double *cell)
-{
-  const int N = h->N, LT = 256 / (N * N);
-  const dim3 grid((h->nz + LT - 1) / LT, h->NF);
-  switch (N) {
-    case 2: k_interp_vort<2><<<grid, 256, 0, h->stream>>>(h->gp, U, h->ointer, OP, cell); break;
-    case 3: k_interp_vort<3><<<grid, 256, 0, h->stream>>>(h->gp, U, h->ointer, OP, cell); break;
-    case 4: k_interp_vort<4><<<grid, 256, 0, h->stream>>>(h->gp, U, h->ointer, OP, cell); break;
-    default: k_interp_vort<5><<<grid, 256, 0, h->stream>>>(h->gp, U, h->ointer, OP, cell); break;
-  }
-}
-
 }  // namespace
 
 int cgd_interpolate(cgd_handle *h, const double *c, const double *rhoc, const double *inter, int32_t OrdPrint,
@@ -1542,7 +1550,11 @@ int cgd_interpolate(cgd_handle *h, const double *c, const double *rhoc, const do
   if (int rc = out_input(h, rhoc, 1, &rd)) return rc;
   const size_t n = out_count(h, OrdPrint);
   if (int rc = out_cells(h, cCell, n, &od)) return rc;
-  k_interp<<<out_blocks(h, OrdPrint), 256, 0, h->stream>>>(h->gp, cd, rd, INTERP_C, h->ointer, OrdPrint, od);
+  CellArgs a{};
+  a.n = 1;
+  a.f[0] = CellOp{rd ? CELL_C_RHO : CELL_C, cd, nullptr, nullptr};
+  a.rho = rd;
+  if (int rc = launch_cells(h, a, OrdPrint, od)) return rc;
   if (od != cCell) CK(cudaMemcpyAsync(cCell, od, n * 8, cudaMemcpyDeviceToHost, h->stream));
   return finish(h);
 }
@@ -1560,7 +1572,10 @@ int cgd_interpolate_wb(cgd_handle *h, const double *u, const double *v, const do
   if (int rc = out_input(h, w, 2, &wd)) return rc;
   const size_t n = out_count(h, OrdPrint);
   if (int rc = out_cells(h, cCell, n, &od)) return rc;
-  k_interp_wb<<<out_blocks(h, OrdPrint), 256, 0, h->stream>>>(h->gp, ud, vd, wd, h->ointer, OrdPrint, od);
+  CellArgs a{};
+  a.n = 1;
+  a.f[0] = CellOp{CELL_WB, wd, ud, vd};
+  if (int rc = launch_cells(h, a, OrdPrint, od)) return rc;
   if (od != cCell) CK(cudaMemcpyAsync(cCell, od, n * 8, cudaMemcpyDeviceToHost, h->stream));
   return finish(h);
 }
@@ -1574,7 +1589,11 @@ int cgd_interpolate_vort(cgd_handle *h, const double *U, const double *inter, in
   if (int rc = stage_in(h, U, h->Ubuf, true, &Ud)) return rc;
   const size_t n = out_count(h, OrdPrint);
   if (int rc = out_cells(h, cCell, n, &od)) return rc;
-  launch_vort(h, Ud, OrdPrint, od);
+  const size_t fs = (size_t)h->nz * h->NumG;
+  CellArgs a{};
+  a.n = 1;
+  a.f[0] = CellOp{CELL_VORT, nullptr, Ud + fs, Ud + 2 * fs};
+  if (int rc = launch_cells(h, a, OrdPrint, od)) return rc;
   if (od != cCell) CK(cudaMemcpyAsync(cCell, od, n * 8, cudaMemcpyDeviceToHost, h->stream));
   return finish(h);
 }
@@ -1596,25 +1615,34 @@ int cgd_output_fields(cgd_handle *h, const double *U, const int32_t *fields, int
   if (int rc = out_cells(h, out, n * nfields, &od)) return rc;
   const size_t fs = (size_t)h->nz * h->NumG;
   const double *rho = Ud, *u = Ud + fs, *v = Ud + 2 * fs, *w = Ud + 3 * fs, *rth = Ud + 4 * fs;
-  const unsigned nb = out_blocks(h, OrdPrint);
-  const double *W = h->ointer;
-  for (int k = 0; k < nfields; ++k) {
-    double *cell = od + (size_t)k * n;
-    const int f = fields[k];
-    switch (f) {
-      case CGD_OUT_RHO: k_interp<<<nb, 256, 0, h->stream>>>(h->gp, rho, nullptr, INTERP_C, W, OrdPrint, cell); break;
-      case CGD_OUT_U: k_interp<<<nb, 256, 0, h->stream>>>(h->gp, u, nullptr, INTERP_C, W, OrdPrint, cell); break;
-      case CGD_OUT_V: k_interp<<<nb, 256, 0, h->stream>>>(h->gp, v, nullptr, INTERP_C, W, OrdPrint, cell); break;
-      case CGD_OUT_WB: k_interp_wb<<<nb, 256, 0, h->stream>>>(h->gp, u, u, w, W, OrdPrint, cell); break;
-      case CGD_OUT_WB_UV: k_interp_wb<<<nb, 256, 0, h->stream>>>(h->gp, u, v, w, W, OrdPrint, cell); break;
-      case CGD_OUT_TH: k_interp<<<nb, 256, 0, h->stream>>>(h->gp, rth, rho, INTERP_POTT, W, OrdPrint, cell); break;
-      case CGD_OUT_PRES: k_interp<<<nb, 256, 0, h->stream>>>(h->gp, rth, nullptr, INTERP_PRES, W, OrdPrint, cell); break;
-      case CGD_OUT_VORT: launch_vort(h, Ud, OrdPrint, cell); break;
-      default:   // tracer ratio rho*q / rho
-        k_interp<<<nb, 256, 0, h->stream>>>(h->gp, Ud + (size_t)(5 + f - CGD_OUT_TR) * fs, rho, INTERP_C, W, OrdPrint,
-                                            cell);
-        break;
+  // up to CELL_MAX quantities, at most one of them the vorticity, per launch
+  for (int k0 = 0; k0 < nfields;) {
+    CellArgs a{};
+    a.rho = rho;
+    a.rhoth = rth;
+    bool vort = false;
+    int k = k0;
+    for (; k < nfields && a.n < CELL_MAX; ++k) {
+      CellOp &f = a.f[a.n];
+      switch (fields[k]) {
+        case CGD_OUT_RHO: f = CellOp{CELL_C, rho, nullptr, nullptr}; break;
+        case CGD_OUT_U: f = CellOp{CELL_C, u, nullptr, nullptr}; break;
+        case CGD_OUT_V: f = CellOp{CELL_C, v, nullptr, nullptr}; break;
+        case CGD_OUT_WB: f = CellOp{CELL_WB, w, u, u}; break;
+        case CGD_OUT_WB_UV: f = CellOp{CELL_WB, w, u, v}; break;
+        case CGD_OUT_TH: f = CellOp{CELL_POTT, nullptr, nullptr, nullptr}; break;
+        case CGD_OUT_PRES: f = CellOp{CELL_PRES, nullptr, nullptr, nullptr}; break;
+        case CGD_OUT_VORT: f = CellOp{CELL_VORT, nullptr, u, v}; break;
+        default:   // tracer ratio rho*q / rho
+          f = CellOp{CELL_C_RHO, Ud + (size_t)(5 + fields[k] - CGD_OUT_TR) * fs, nullptr, nullptr};
+          break;
+      }
+      if (f.op == CELL_VORT && vort) break;   // the next launch's
+      vort = vort || f.op == CELL_VORT;
+      ++a.n;
     }
+    if (int rc = launch_cells(h, a, OrdPrint, od + (size_t)k0 * n)) return rc;
+    k0 = k;
   }
   if (od != out) CK(cudaMemcpyAsync(out, od, n * nfields * 8, cudaMemcpyDeviceToHost, h->stream));
   return finish(h);
