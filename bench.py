@@ -635,8 +635,8 @@ def ensemble_measure(K, warmup, rank, ranks, torch):
             "mass_drift_fp64_max": float(max(abs(x) for x in res["fp64"]["drift"])),
             "finite": res["fp64"]["finite"] and res["mixed"]["finite"],
             "perturbation": f"theta +-{E['theta_amp']} K, u,v +-{E['wind_amp']} m/s, seed {E['seed0']}+member",
-            "gpu_launches": {"fused": 3, "members": 15 * len(members)}.get(
-                res["fp64"]["tuning"].split("stage=")[1].split(";")[0], 15) * K}
+            "gpu_launches": {"fused": 3, "members": 9 * len(members)}.get(
+                res["fp64"]["tuning"].split("stage=")[1].split(";")[0], 9) * K}
 
 
 def run_ensemble(args, rank, world, local):
@@ -658,7 +658,7 @@ def run_ensemble(args, rank, world, local):
             "warmup": args.warmup, "ms_per_step": r["ms_per_step"], "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64", "data": "synthetic (baroclinic wave + seeded member perturbations)",
             "config": {"workload": "batched ensemble: 48 members on 3 grids, one CUDA graph per ensemble step "
-                                   "(15 launches split, or 3 fused persistent stage launches; the autotuner picks "
+                                   "(9 launches split, or 3 fused persistent stage launches; the autotuner picks "
                                    "the work-list order, the form and the levels per phase-2 CTA)",
                        "grids": r["grids"], "per_grid": r["per_grid"], "dt": r["dt"], "hours": r["hours"],
                        "steps_total": r["steps_total"], "perturbation": r["perturbation"],
@@ -836,7 +836,7 @@ def run_ours(args, cfg, rank, world, local):
             "adjoint": adjoint,
             "ensemble": ensemble,
             "output": outp,
-            "gpu_launches": 15 * args.steps,
+            "gpu_launches": 9 * args.steps,
             "cpu_baseline": cpu,
             "clocks": clk,
         }
@@ -912,7 +912,7 @@ def run_shard(args, cfg, rank, world, local):
                 "e2e": {"value": Ke / te, "unit": UNIT, "h2d_bytes_per_step": tot_bytes,
                         "d2h_bytes_per_step": tot_bytes, "steps": Ke,
                         "call": "cgd_ros_step(h_rank, host_part, dt, 1) per step on every rank"},
-                "gpu_launches": (15 + (12 if world > 1 else 0)) * args.steps, "clocks": clk}
+                "gpu_launches": (9 + (12 if world > 1 else 0)) * args.steps, "clocks": clk}
         print(json.dumps(line), flush=True)
     d.close()
     if world > 1:

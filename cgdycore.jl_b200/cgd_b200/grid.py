@@ -579,6 +579,18 @@ class Grid:
     M: np.ndarray
     MMass: np.ndarray
     dz: np.ndarray
+    layers: np.ndarray = None   # a part of a decomposed grid: layer_ratios of the whole grid
+
+
+def layer_ratios(grid):
+    """The layer-thickness ratios z(l) / z(0) (nz) of the grid's first element:
+    the sum of J's first node over the element's nodes, in node order (the
+    library's own choice for a whole grid, cgd_set_layers)."""
+    J = grid.J[:, 0, :, 0]
+    a = np.zeros(J.shape[1])
+    for ID in range(J.shape[0]):
+        a = a + J[ID]
+    return a / a[0]
 
 
 def init_grid_sphere(nPanel, OrdPoly, z, H, Rad):

@@ -136,6 +136,9 @@ class Dycore:
         _lib.check(rc, "cgd_create")
         self._xfn = None
         self.h = h
+        if getattr(grid, "layers", None) is not None:
+            z = np.ascontiguousarray(grid.layers, np.float64)
+            _lib.check(L.cgd_set_layers(h, z.ctypes.data), "cgd_set_layers")
         self._mmass = grid.MMass if hasattr(grid.MMass, "data_ptr") else np.asfortranarray(grid.MMass)
 
     def set_physics(self, held_suarez=None, damping=None):

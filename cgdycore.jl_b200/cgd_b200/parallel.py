@@ -28,7 +28,7 @@ from dataclasses import dataclass
 
 import numpy as np
 
-from .grid import Grid, inverse_map
+from .grid import Grid, inverse_map, layer_ratios
 
 
 def partition_elements(NF, nranks):
@@ -108,7 +108,7 @@ class HaloPlan:
                     np.asfortranarray(self.glob), grid.faces[e], grid.xw, grid.w, grid.DS, grid.DW,
                     np.asfortranarray(grid.X[..., e]), np.asfortranarray(grid.dXdxI[..., e]),
                     np.asfortranarray(grid.J[..., e]), np.asfortranarray(grid.M[:, d, :]), mm,
-                    np.asfortranarray(grid.dz[:, d]))
+                    np.asfortranarray(grid.dz[:, d]), layer_ratios(grid))
 
     def restrict(self, U):
         """The rank's part of a global state (nz, NumG, NV)."""

@@ -8,6 +8,7 @@
 #include "../../include/cgd_b200.h"
 #include "cgd_kernels.cuh"
 #include "cgd_phase2.cuh"
+#include "cgd_flat.cuh"
 #include "cgd_batch.cuh"
 #include "cgd_init.cuh"
 #include "cgd_output.cuh"
@@ -29,7 +30,7 @@ using namespace cgd;
 
 namespace {
 
-constexpr int NPROF = 15;   // kernels per step whose durations are recorded
+constexpr int NPROF = 9;   // kernels per step whose durations are recorded
 
 struct Buf {
   void *p = nullptr;
@@ -63,13 +64,17 @@ struct cgd_handle {
   cudaEvent_t order_ev = nullptr;
   std::vector<Buf> bufs;
   double *met = nullptr, *M = nullptr, *dz = nullptr;
+  double *hm = nullptr, *zl = nullptr;   // factors of a flat product grid (GP::hm, GP::zl)
   int *glob = nullptr, *inv_ptr = nullptr;
+  int4 *etab = nullptr;
+  unsigned char *own = nullptr;
   long long *inv_off = nullptr, *inv_tab = nullptr;
-  double *C = nullptr, *T1 = nullptr, *Vst = nullptr, *k1 = nullptr, *k2 = nullptr;
+  // element contributions of phase 1 and of phase 2
+  double *C1 = nullptr, *C = nullptr, *Vst = nullptr, *k1 = nullptr, *k2 = nullptr;
   double *Ubuf = nullptr, *Fbuf = nullptr, *bands = nullptr, *part = nullptr, *scal = nullptr;
   double *jbg = nullptr;   // Jacobian bands of the current step, [8][NumG][nz-1]
-  double *pres = nullptr, *pres_st = nullptr;   // pressure of the state and of the stage state
-  double *aLF = nullptr, *aLU = nullptr, *aLT1 = nullptr;   // adjoint buffers (allocated on first use)
+  double *pres = nullptr;  // pressure of the stage state
+  double *aLF = nullptr, *aLU = nullptr, *aLT1 = nullptr, *aT1 = nullptr;   // adjoint buffers (allocated on first use)
   // step adjoint workspace: stage states, stage tendencies, k adjoints, ...
   double *aLk[2] = {}, *aAR = nullptr, *aLV = nullptr, *aLt = nullptr;
   StepTape work_tape;              // cgd_ros_step_adjoint's own replay
@@ -189,7 +194,7 @@ GP ranged_gp(const cgd_handle *h, int &nIF)
 }
 
 template <int N, int NT, typename R>
-void launch_hv1r(cgd_handle *h, const double *U, double *C)
+void launch_hv1r(cgd_handle *h, const double *U, double *C, double *Pr)
 {
   using T = HV1Tile<N, R>;
   constexpr size_t smem = HV1Smem<N, NT, R, T::LT>::BYTES;
@@ -200,30 +205,39 @@ void launch_hv1r(cgd_handle *h, const double *U, double *C)
   const GP gp = ranged_gp(h, nIF);
   if (nIF <= 0) return;
   dim3 grid((h->nz + T::LT - 1) / T::LT, nIF);   // the level tiles of one element run back to back
-  k_hypervisc1<N, NT, R><<<grid, T::THREADS, smem, h->stream>>>(gp, U, C);
+#ifdef CGD_FAST
+  if (gp.flat) {
+    static std::atomic<unsigned long long> fattr{0};
+    if (first_on_device(fattr))
+      cudaFuncSetAttribute(k_hypervisc1_flat<N, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_hypervisc1_flat<N, NT, R><<<grid, T::THREADS, smem, h->stream>>>(gp, U, C, Pr);
+    return;
+  }
+#endif
+  k_hypervisc1<N, NT, R><<<grid, T::THREADS, smem, h->stream>>>(gp, U, C, Pr);
 }
 
 template <int N, int NT>
-void launch_hv1t(cgd_handle *h, const double *U, double *C)
+void launch_hv1t(cgd_handle *h, const double *U, double *C, double *Pr)
 {
-  if (h->mix) launch_hv1r<N, NT, float>(h, U, C);
-  else launch_hv1r<N, NT, double>(h, U, C);
+  if (h->mix) launch_hv1r<N, NT, float>(h, U, C, Pr);
+  else launch_hv1r<N, NT, double>(h, U, C, Pr);
 }
 
 template <int N>
-void launch_hv1(cgd_handle *h, const double *U, double *C)
+void launch_hv1(cgd_handle *h, const double *U, double *C, double *Pr)
 {
   switch (h->NumTr) {
-    case 0: launch_hv1t<N, 0>(h, U, C); break;
-    case 1: launch_hv1t<N, 1>(h, U, C); break;
-    case 2: launch_hv1t<N, 2>(h, U, C); break;
-    case 3: launch_hv1t<N, 3>(h, U, C); break;
-    default: launch_hv1t<N, 4>(h, U, C); break;
+    case 0: launch_hv1t<N, 0>(h, U, C, Pr); break;
+    case 1: launch_hv1t<N, 1>(h, U, C, Pr); break;
+    case 2: launch_hv1t<N, 2>(h, U, C, Pr); break;
+    case 3: launch_hv1t<N, 3>(h, U, C, Pr); break;
+    default: launch_hv1t<N, 4>(h, U, C, Pr); break;
   }
 }
 
 template <int N, int NT, typename R>
-void launch_p2r(cgd_handle *h, const double *U, const double *Pr, const double *T1, double *C)
+void launch_p2r(cgd_handle *h, const double *U, const double *Pr, const double *C1, double *C)
 {
   using CF = P2Cfg<N, NT, R>;
   static std::atomic<unsigned long long> attr{0};
@@ -234,52 +248,58 @@ void launch_p2r(cgd_handle *h, const double *U, const double *Pr, const double *
   const GP gp = ranged_gp(h, nIF);
   if (nIF <= 0) return;
   dim3 grid(p2_items<CF>(h->nz), nIF);   // the items of one element run back to back
-  k_phase2<N, NT, R><<<grid, CF::THREADS, CF::SMEM, h->stream>>>(gp, U, Pr, T1, C);
+#ifdef CGD_FAST
+  if (gp.flat) {
+    using FF = P2Flat<N, NT, R>;
+    static std::atomic<unsigned long long> fattr{0};
+    if (first_on_device(fattr))
+      cudaFuncSetAttribute(k_phase2_flat<N, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FF::SMEM);
+    k_phase2_flat<N, NT, R><<<grid, FF::THREADS, FF::SMEM, h->stream>>>(gp, U, Pr, C1, C);
+    return;
+  }
+#endif
+  k_phase2<N, NT, R><<<grid, CF::THREADS, CF::SMEM, h->stream>>>(gp, U, Pr, C1, C);
 }
 
 template <int N, int NT>
-void launch_p2(cgd_handle *h, const double *U, const double *Pr, const double *T1, double *C)
+void launch_p2(cgd_handle *h, const double *U, const double *Pr, const double *C1, double *C)
 {
-  if (h->mix) launch_p2r<N, NT, float>(h, U, Pr, T1, C);
-  else launch_p2r<N, NT, double>(h, U, Pr, T1, C);
+  if (h->mix) launch_p2r<N, NT, float>(h, U, Pr, C1, C);
+  else launch_p2r<N, NT, double>(h, U, Pr, C1, C);
 }
 
 template <int N>
-void launch_p2(cgd_handle *h, const double *U, const double *Pr, const double *T1, double *C)
+void launch_p2(cgd_handle *h, const double *U, const double *Pr, const double *C1, double *C)
 {
   switch (h->NumTr) {
-    case 0: launch_p2<N, 0>(h, U, Pr, T1, C); break;
-    case 1: launch_p2<N, 1>(h, U, Pr, T1, C); break;
-    case 2: launch_p2<N, 2>(h, U, Pr, T1, C); break;
-    case 3: launch_p2<N, 3>(h, U, Pr, T1, C); break;
-    default: launch_p2<N, 4>(h, U, Pr, T1, C); break;
+    case 0: launch_p2<N, 0>(h, U, Pr, C1, C); break;
+    case 1: launch_p2<N, 1>(h, U, Pr, C1, C); break;
+    case 2: launch_p2<N, 2>(h, U, Pr, C1, C); break;
+    case 3: launch_p2<N, 3>(h, U, Pr, C1, C); break;
+    default: launch_p2<N, 4>(h, U, Pr, C1, C); break;
   }
 }
 
-void hv1(cgd_handle *h, const double *U, double *C)
+// Phase 1 -> C, and the pressure of U -> Pr (unless null).
+void hv1(cgd_handle *h, const double *U, double *C, double *Pr)
 {
   switch (h->N) {
-    case 2: launch_hv1<2>(h, U, C); break;
-    case 3: launch_hv1<3>(h, U, C); break;
-    case 4: launch_hv1<4>(h, U, C); break;
-    default: launch_hv1<5>(h, U, C); break;
+    case 2: launch_hv1<2>(h, U, C, Pr); break;
+    case 3: launch_hv1<3>(h, U, C, Pr); break;
+    case 4: launch_hv1<4>(h, U, C, Pr); break;
+    default: launch_hv1<5>(h, U, C, Pr); break;
   }
 }
 
-void phase2(cgd_handle *h, const double *U, const double *Pr, const double *T1, double *C)
+// Phase 2 of U with pressure Pr and the phase-1 contributions C1 -> C.
+void phase2(cgd_handle *h, const double *U, const double *Pr, const double *C1, double *C)
 {
   switch (h->N) {
-    case 2: launch_p2<2>(h, U, Pr, T1, C); break;
-    case 3: launch_p2<3>(h, U, Pr, T1, C); break;
-    case 4: launch_p2<4>(h, U, Pr, T1, C); break;
-    default: launch_p2<5>(h, U, Pr, T1, C); break;
+    case 2: launch_p2<2>(h, U, Pr, C1, C); break;
+    case 3: launch_p2<3>(h, U, Pr, C1, C); break;
+    case 4: launch_p2<4>(h, U, Pr, C1, C); break;
+    default: launch_p2<5>(h, U, Pr, C1, C); break;
   }
-}
-
-void pressure(cgd_handle *h, const double *U, double *p)
-{
-  const long long n = (long long)h->nz * h->NumG;
-  k_pressure<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->gp, U, p);
 }
 
 // The column physics added to a tendency (no launch when none is set).
@@ -290,21 +310,18 @@ void physics(cgd_handle *h, const double *U, const double *p, double *F)
   k_physics<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->gp, U, p, F);
 }
 
-// wsplit: the phase-2 tendency (w split into two contributions, FP64 output);
-// otherwise phase 1, whose output is the cache (stored like the contributions)
-// or, with tendency_out, an FP64 array for the caller.
-void gather(cgd_handle *h, const double *C, double *out, bool wsplit, bool tendency_out = false)
+// The DSS: wsplit for the phase-2 tendency (w in two contributions), otherwise
+// the phase-1 cache.
+void gather(cgd_handle *h, const double *C, double *out, bool wsplit)
 {
   long long n = (long long)h->nz * h->NumG;
   const unsigned nb = (unsigned)((n + 255) / 256);
   if (h->mix) {
-    if (wsplit) k_gather<true, false, true><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
-    else if (tendency_out) k_gather<false, false, true><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
-    else k_gather<false, true, true><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
+    if (wsplit) k_gather<true, true><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
+    else k_gather<false, true><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
   } else {
-    if (wsplit) k_gather<true, false, false><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
-    else if (tendency_out) k_gather<false, false, false><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
-    else k_gather<false, true, false><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
+    if (wsplit) k_gather<true, false><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
+    else k_gather<false, false><<<nb, 256, 0, h->stream>>>(h->gp, C, out);
   }
 }
 
@@ -371,48 +388,35 @@ ColArgs step_args(cgd_handle *h, double *U, double dt)
   return a;
 }
 
-// The three pieces of a Rosenbrock-W stage, split at the two direct-stiffness
-// summations (where a decomposed grid exchanges element contributions):
-//   piece 0: (stage 1: the pressure of the step's state) phase 1 -> C
-//   piece 1: DSS of phase 1 -> T1, phase 2 -> C
-//   piece 2: column stage (DSS of phase 2, solve, update), then the pressure
-//            of the next stage state
+// The three pieces of a Rosenbrock-W stage (at the two direct-stiffness
+// summations a decomposed grid exchanges element contributions):
+//   piece 0: phase 1 -> C1, and the pressure of the stage state
+//   piece 1: phase 2, summing C1 -> C
+//   piece 2: column stage (DSS of phase 2, solve, update)
 // e counts the profiling events of the single-process step.
 void stage_piece(cgd_handle *h, double *U, const ColArgs &a0, int stage, int piece, int &e)
 {
   const double *Vsrc = stage == 0 ? U : h->Vst;
   if (piece == 0) {
-    if (stage == 0) {
-      pressure(h, U, h->pres);
-      rec(h, e++);
-    }
-    hv1(h, Vsrc, h->C);
-    rec(h, e++);
+    hv1(h, Vsrc, h->C1, h->pres);
   } else if (piece == 1) {
-    gather(h, h->C, h->T1, false);
-    rec(h, e++);
-    phase2(h, Vsrc, stage == 0 ? h->pres : h->pres_st, h->T1, h->C);
-    rec(h, e++);
+    phase2(h, Vsrc, h->pres, h->C1, h->C);
   } else {
     ColArgs a = a0;
     a.Vs = Vsrc;
-    a.ps = stage == 0 ? h->pres : h->pres_st;
+    a.ps = h->pres;
     if (stage == 0) {
       a.kout = h->k1; a.Vout = h->Vst;
       column<0>(h, a);
-      rec(h, e++);
-      pressure(h, h->Vst, h->pres_st);
     } else if (stage == 1) {
       a.kout = h->k2; a.Vout = h->Vst;
       column<1>(h, a);
-      rec(h, e++);
-      pressure(h, h->Vst, h->pres_st);
     } else {
       a.kout = nullptr; a.Vout = U;
       column<2>(h, a);
     }
-    rec(h, e++);
   }
+  rec(h, e++);
 }
 
 // One SSP-Knoth step on device state U (in place).
@@ -454,16 +458,16 @@ __global__ void __launch_bounds__(256) k_halo_unpack(const double *__restrict__ 
   C[(((size_t)pe * NC + f) * DoF + node) * nz + l] = rbuf[t];
 }
 
-void halo_pack(cgd_handle *h, int nf)
+void halo_pack(cgd_handle *h, const double *C, int nf)
 {
   const long long n = (long long)h->nsend * nf * h->nz;
-  if (n) k_halo_pack<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->C, h->sbuf, h->send_list, h->nsend, nf,
+  if (n) k_halo_pack<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(C, h->sbuf, h->send_list, h->nsend, nf,
                                                                          h->DoF, h->NV + 1, h->nz);
 }
-void halo_unpack(cgd_handle *h, int nf)
+void halo_unpack(cgd_handle *h, double *C, int nf)
 {
   const long long n = (long long)h->nghost * nf * h->nz;
-  if (n) k_halo_unpack<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->rbuf, h->C, h->nghost, h->NF, nf,
+  if (n) k_halo_unpack<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->rbuf, C, h->nghost, h->NF, nf,
                                                                            h->DoF, h->NV + 1, h->nz);
 }
 
@@ -526,11 +530,13 @@ int part_pieces(cgd_handle *const *parts, int n, double *const *U, double dt, bo
     CK(cudaEventCreateWithFlags(&h0->xa, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&h0->xb, cudaEventDisableTiming));
   }
+  // the contribution buffer of the DSS point with nf fields
+  auto buf = [&](int r, int nf) { return nf == nf1 ? parts[r]->C1 : parts[r]->C; };
   auto xchg = [&](int nf) -> int {
-    for (int r = 0; r < n; ++r) halo_pack(parts[r], nf);
+    for (int r = 0; r < n; ++r) halo_pack(parts[r], buf(r, nf), nf);
     int rc = n > 1 ? group_exchange(parts, n, nf, h0->stream) : callback_exchange(h0, nf);
     if (rc) return rc;
-    for (int r = 0; r < n; ++r) halo_unpack(parts[r], nf);
+    for (int r = 0; r < n; ++r) halo_unpack(parts[r], buf(r, nf), nf);
     return CGD_OK;
   };
   // kern(r) launches part r's phase-1 or phase-2 kernel on its stream over
@@ -563,13 +569,8 @@ int part_pieces(cgd_handle *const *parts, int n, double *const *U, double dt, bo
     return CGD_OK;
   };
   if (rhs_only) {
-    if (int rc = split(nf1, [&](int r) { hv1(parts[r], U[r], parts[r]->C); })) return rc;
-    for (int r = 0; r < n; ++r) {
-      cgd_handle *q = parts[r];
-      gather(q, q->C, q->T1, false);
-      pressure(q, U[r], q->pres);
-    }
-    if (int rc = split(nf2, [&](int r) { phase2(parts[r], U[r], parts[r]->pres, parts[r]->T1, parts[r]->C); }))
+    if (int rc = split(nf1, [&](int r) { hv1(parts[r], U[r], parts[r]->C1, parts[r]->pres); })) return rc;
+    if (int rc = split(nf2, [&](int r) { phase2(parts[r], U[r], parts[r]->pres, parts[r]->C1, parts[r]->C); }))
       return rc;
     for (int r = 0; r < n; ++r) {
       gather(parts[r], parts[r]->C, F[r], true);
@@ -582,15 +583,9 @@ int part_pieces(cgd_handle *const *parts, int n, double *const *U, double dt, bo
   int e = 0;
   for (int stage = 0; stage < 3; ++stage) {
     auto vsrc = [&](int r) -> const double * { return stage == 0 ? U[r] : parts[r]->Vst; };
-    if (stage == 0)
-      for (int r = 0; r < n; ++r) pressure(parts[r], U[r], parts[r]->pres);
-    if (int rc = split(nf1, [&](int r) { hv1(parts[r], vsrc(r), parts[r]->C); })) return rc;
-    for (int r = 0; r < n; ++r) gather(parts[r], parts[r]->C, parts[r]->T1, false);
-    auto p2 = [&](int r) {
-      cgd_handle *q = parts[r];
-      phase2(q, vsrc(r), stage == 0 ? q->pres : q->pres_st, q->T1, q->C);
-    };
-    if (int rc = split(nf2, p2)) return rc;
+    if (int rc = split(nf1, [&](int r) { hv1(parts[r], vsrc(r), parts[r]->C1, parts[r]->pres); })) return rc;
+    if (int rc = split(nf2, [&](int r) { phase2(parts[r], vsrc(r), parts[r]->pres, parts[r]->C1, parts[r]->C); }))
+      return rc;
     for (int r = 0; r < n; ++r) stage_piece(parts[r], U[r], a[r], stage, 2, e);
   }
   return CGD_OK;
@@ -603,6 +598,31 @@ void ensure_ref(cgd_handle *h, const double *Ud)
   k_refprof<<<h->nz, 256, 0, h->stream>>>(h->gp, Ud, h->pref, h->thref);
   h->have_ref = true;
 }
+
+#ifdef CGD_FAST
+// The factors of a flat product grid (zin: the layers' z on the host, else from
+// the first element), and whether the grid is one.
+int flat_factors(cgd_handle *h, const double *zin)
+{
+  GP &P = h->gp;
+  const long long n = (long long)h->NF * h->DoF * h->nz;
+  int bad = 1;
+  double *zd = nullptr;
+  if (zin) {
+    zd = h->part;
+    CK(cudaMemcpyAsync(zd, zin, h->nz * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  }
+  CK(cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
+  k_flat_layers<<<1, 64, 0, h->stream>>>(P, zd, h->zl);
+  k_flat_factors<<<h->NF, 32, 0, h->stream>>>(P, h->hm);
+  k_flat_check<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(P, std::fabs(2.0 * h->cfg.Omega), h->flag);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(&bad, h->flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  P.flat = !bad;
+  return CGD_OK;
+}
+#endif
 
 void free_graph(cgd_handle *h)
 {
@@ -856,15 +876,29 @@ static int create_impl(const cgd_config *cfg, const int64_t *glob, const double 
     if (ptr[g + 1] - ptr[g] <= 4)
       for (int q = ptr[g]; q < ptr[g + 1]; ++q) tab[(size_t)4 * g + (q - ptr[g])] = off[q];
   TRY(dalloc(h, &h->inv_tab, tab.size()));
+  // the same rows per element node (offsets in units of nz), and the first
+  // local contributor of every DOF (it writes the DOF's pressure)
+  std::vector<int4> etab((size_t)DoF * NF);
+  std::vector<unsigned char> own((size_t)DoF * NF, 0);
+  std::vector<unsigned char> seen(NumG, 0);
+  for (size_t i = 0; i < etab.size(); ++i) {
+    const int g = glob0[i];
+    const long long *r = &tab[(size_t)4 * g];
+    auto at = [&](int k) { return r[k] < 0 ? -1 : (int)(r[k] / nz); };
+    etab[i] = int4{at(0), at(1), at(2), at(3)};
+    if (!seen[g]) own[i] = seen[g] = 1;
+  }
+  TRY(dalloc(h, &h->etab, etab.size()));
+  TRY(dalloc(h, &h->own, own.size()));
   // contribution buffer: the local elements, then the ghost pseudo-elements
   const size_t ghost_elems = ((size_t)nghost + DoF - 1) / DoF;
   TRY(dalloc(h, &h->C, ENL * (NV + 1) + ghost_elems * DoF * nz * (NV + 1)));
+  TRY(dalloc(h, &h->C1, ENL * (NV + 1) + ghost_elems * DoF * nz * (NV + 1)));
   if (halo) {
     TRY(dalloc(h, &h->send_list, (size_t)std::max(nsend, 1)));
     TRY(dalloc(h, &h->sbuf, (size_t)std::max(nsend, 1) * (NV + 1) * nz));
     TRY(dalloc(h, &h->rbuf, (size_t)std::max(nghost, 1) * (NV + 1) * nz));
   }
-  TRY(dalloc(h, &h->T1, S * NV));
   TRY(dalloc(h, &h->Vst, S * NV));
   TRY(dalloc(h, &h->k1, S * NV));
   TRY(dalloc(h, &h->k2, S * NV));
@@ -873,7 +907,6 @@ static int create_impl(const cgd_config *cfg, const int64_t *glob, const double 
   TRY(dalloc(h, &h->bands, 8 * (size_t)(nz - 1) * NumG));
   TRY(dalloc(h, &h->jbg, 8 * (size_t)(nz - 1) * NumG));
   TRY(dalloc(h, &h->pres, S));
-  TRY(dalloc(h, &h->pres_st, S));
   h->mix = cfg->precision == CGD_PREC_MIXED;
   TRY(dalloc(h, &h->pref, nz));
   TRY(dalloc(h, &h->thref, nz));
@@ -892,6 +925,7 @@ static int create_impl(const cgd_config *cfg, const int64_t *glob, const double 
   if ((!dev_metric && up(h->met, met.data(), met.size() * 8)) || cudaGetLastError() != cudaSuccess || up(h->M, M, 2 * S * 8) || up(h->dz, dz, S * 8) ||
       up(h->glob, glob0.data(), glob0.size() * 4) || up(h->inv_ptr, ptr.data(), ptr.size() * 4) ||
       up(h->inv_off, off.data(), off.size() * 8) || up(h->inv_tab, tab.data(), tab.size() * 8) ||
+      up(h->etab, etab.data(), etab.size() * sizeof(int4)) || up(h->own, own.data(), own.size()) ||
       (halo && nsend && up(h->send_list, halo->send_list, (size_t)nsend * 4))) {
     cudaError_t e = cudaGetLastError();
     cuda_fail(h, e, "cgd_create upload");
@@ -908,12 +942,24 @@ static int create_impl(const cgd_config *cfg, const int64_t *glob, const double 
   GP &P = h->gp;
   P.N = N; P.DoF = DoF; P.nz = nz; P.NF = NF; P.NumG = NumG; P.NumTr = h->NumTr; P.NV = NV; P.NC = NV + 1;
   P.met = h->met; P.M = h->M; P.dz = h->dz; P.glob = h->glob; P.inv_ptr = h->inv_ptr; P.inv_off = h->inv_off;
-  P.inv_tab = h->inv_tab;
+  P.inv_tab = h->inv_tab; P.etab = h->etab; P.own = h->own;
   P.pref = h->pref; P.thref = h->thref;
   for (int i = 0; i < 25; ++i) { P.D[i] = 0.0; P.DW[i] = 0.0; }
   for (int i = 0; i < N * N; ++i) { P.D[i] = DS[i]; P.DW[i] = DW[i]; }
   P.Grav = cfg->Grav; P.Rd = cfg->Rd; P.p0 = cfg->p0; P.kappa = cfg->Rd / cfg->Cpd;
   P.nuCurl = cfg->HyperDCurl; P.nuGrad = cfg->HyperDGrad; P.nuDiv = cfg->HyperDDiv;
+
+  P.flat = 0;
+#ifdef CGD_FAST
+  {
+    double *hm = nullptr;
+    const size_t nh = (size_t)NF * H_N * DoF;
+    TRY(dalloc(h, &hm, nh + (size_t)(6 + 2 * N) * nz));
+    P.hm = h->hm = hm;
+    P.zl = h->zl = hm + nh;
+    TRY(flat_factors(h, nullptr));
+  }
+#endif
 
   // SSP-Knoth: a = alpha/Gamma, c = -inv(Gamma), m = Gamma'\b (RosenbrockMethod.jl:26-47)
   RK &r = h->rk;
@@ -1008,8 +1054,8 @@ int cgd_hypervisc_phase1(cgd_handle *h, const double *U, double *Temp1)
   bool tdev = is_device_ptr(Temp1);
   double *td = tdev ? Temp1 : h->Fbuf;
   ensure_ref(h, Ud);
-  hv1(h, Ud, h->C);
-  gather(h, h->C, td, false, true);
+  hv1(h, Ud, h->C1, nullptr);
+  gather(h, h->C1, td, false);
   if (!tdev)
     CK(cudaMemcpyAsync(Temp1, td, (size_t)h->nz * h->NumG * h->NV * 8, cudaMemcpyDeviceToHost, h->stream));
   return finish(h);
@@ -1030,10 +1076,8 @@ int cgd_rhs(cgd_handle *h, const double *U, double *F)
     if (!fdev) CK(cudaMemcpyAsync(F, fd, (size_t)h->nz * h->NumG * h->NV * 8, cudaMemcpyDeviceToHost, h->stream));
     return finish(h);
   }
-  hv1(h, Ud, h->C);
-  gather(h, h->C, h->T1, false);
-  pressure(h, Ud, h->pres);
-  phase2(h, Ud, h->pres, h->T1, h->C);
+  hv1(h, Ud, h->C1, h->pres);
+  phase2(h, Ud, h->pres, h->C1, h->C);
   gather(h, h->C, fd, true);
   physics(h, Ud, h->pres, fd);
   if (!fdev) CK(cudaMemcpyAsync(F, fd, (size_t)h->nz * h->NumG * h->NV * 8, cudaMemcpyDeviceToHost, h->stream));
@@ -1335,6 +1379,18 @@ int cgd_mass_dz(int32_t OrdPoly, int32_t nz, int32_t NF, int32_t NumG, const int
   }
   cudaFree(dptr);
   if (e != cudaSuccess) return cuda_fail(h, e, "cgd_mass_dz");
+  return CGD_OK;
+}
+
+int cgd_set_layers(cgd_handle *h, const double *z)
+{
+  if (!h || !z) return CGD_ERR_INVALID_ARG;
+  for (int l = 0; l < h->nz; ++l)
+    if (!(z[l] > 0.0)) return CGD_ERR_INVALID_ARG;
+#ifdef CGD_FAST
+  if (int rc = flat_factors(h, z)) return rc;
+  free_graph(h);
+#endif
   return CGD_OK;
 }
 
@@ -1713,7 +1769,8 @@ int adjoint_alloc(cgd_handle *h, bool step)
   const size_t S = (size_t)h->nz * h->NumG, SV = S * h->NV;
   int rc = CGD_OK;
   if (!h->aLF) {
-    rc = dalloc(h, &h->aLF, SV);
+    rc = dalloc(h, &h->aT1, SV);
+    if (!rc) rc = dalloc(h, &h->aLF, SV);
     if (!rc) rc = dalloc(h, &h->aLU, SV);
     if (!rc) rc = dalloc(h, &h->aLT1, S * 5);
   }
@@ -1734,10 +1791,9 @@ int rhs_adjoint_core(cgd_handle *h, const double *Ud, const double *LFd, double 
 {
   const size_t S = (size_t)h->nz * h->NumG;
   if (!T1) {
-    hv1(h, Ud, h->C);
-    gather(h, h->C, h->T1, false);
-    pressure(h, Ud, h->pres);
-    T1 = h->T1;
+    hv1(h, Ud, h->C1, h->pres);
+    gather(h, h->C1, h->aT1, false);
+    T1 = h->aT1;
     pres = h->pres;
   }
   CK(cudaMemsetAsync(LUd, 0, S * h->NV * 8, h->stream));
@@ -1801,10 +1857,9 @@ int record_step(cgd_handle *h, StepTape &t, const double *u0, double dt, double 
   a.jbg = t.jbg;
   const double *Vs[3] = {t.u0, t.V2, t.V3};
   for (int st = 0; st < 3; ++st) {
-    hv1(h, Vs[st], h->C);
-    gather(h, h->C, t.T1[st], false);
-    pressure(h, Vs[st], t.P[st]);
-    phase2(h, Vs[st], t.P[st], t.T1[st], h->C);
+    hv1(h, Vs[st], h->C1, t.P[st]);
+    gather(h, h->C1, t.T1[st], false);
+    phase2(h, Vs[st], t.P[st], h->C1, h->C);
     a.kout = t.k[st];
     if (st == 0) { a.Vout = t.V2; column<0>(h, a); }
     else if (st == 1) { a.Vout = t.V3; column<1>(h, a); }
@@ -1988,9 +2043,8 @@ int cgd_kernel_times(cgd_handle *h, char *names, int32_t names_len, double *ms, 
 {
   if (!h || !ms) return CGD_ERR_INVALID_ARG;
   if (!h->profile) return CGD_ERR_UNSUPPORTED;
-  static const char *nm[NPROF] = {"pressure", "hypervisc1", "gather", "phase2", "column", "pressure",
-                                  "hypervisc1", "gather", "phase2", "column", "pressure",
-                                  "hypervisc1", "gather", "phase2", "column"};
+  static const char *nm[NPROF] = {"hypervisc1", "phase2", "column", "hypervisc1", "phase2",
+                                  "column", "hypervisc1", "phase2", "column"};
   std::string all;
   int n = nmax < NPROF ? nmax : NPROF;
   for (int i = 0; i < n; ++i) {
@@ -2013,15 +2067,9 @@ int cgd_kernel_times(cgd_handle *h, char *names, int32_t names_len, double *ms, 
 }  // extern "C"
 
 // ===========================================================================
-// Batched ensemble (cgd_batch_*): the members' steps as one graph of 15
+// Batched ensemble (cgd_batch_*): the members' steps as one graph of 9
 // launches over flat work lists.
 // ===========================================================================
-// Work lists of an ensemble: 0 phase-1 tiles of 256/N^2 levels, 1 column-level
-// blocks of 256 (pressure, gather), 2 phase-2 items, 3 column blocks, 4 phase-2
-// items of the fused form and of the 8-level split form, 5 phase-1 tiles of the split form (HV1Tile: 16
-// levels at p = 4 in FP64, else as list 0)
-constexpr int BATCH_LISTS = 6;
-
 struct cgd_batch {
   std::vector<cgd_handle *> mem;
   int N = 0, NT = 0, nzmax = 0;
@@ -2030,7 +2078,7 @@ struct cgd_batch {
   cudaStream_t stream = nullptr;
   cudaEvent_t order_ev = nullptr;   // orders a step after the first member's caller stream
   // work lists, one set per candidate order; a candidate is (order, form):
-  // candidate c runs order c % NORD in form c / NORD: split into 15 launches
+  // candidate c runs order c % NORD in form c / NORD: split into 9 launches
   // (FORM_SPLIT), split with phase 2 in 8-level CTAs (FORM_SPLIT8, p = 4),
   // as three fused stage launches (FORM_FUSED), or every member's own
   // single-member step on its own stream inside the graph (FORM_MEMBERS;
@@ -2039,8 +2087,8 @@ struct cgd_batch {
   static constexpr int NORD = 3;
   static constexpr int FORM_SPLIT = 0, FORM_SPLIT8 = 1, FORM_FUSED = 2, FORM_MEMBERS = 3, NFORM = 4;
   static constexpr int NCAND = NFORM * NORD;
-  WItem *w[NORD][BATCH_LISTS] = {};
-  int n[BATCH_LISTS] = {};
+  WItem *w[NORD][WL_N] = {};
+  int n[WL_N] = {};
   cudaGraph_t graph[NCAND] = {};
   cudaGraphExec_t gexec[NCAND] = {};
   bool use[NCAND] = {};
@@ -2048,11 +2096,11 @@ struct cgd_batch {
   bool tuned = false, autotune = false;
   double tune_ms[NCAND] = {};
   // fused form: grid (CTAs resident on the device), dynamic shared memory,
-  // barrier state, second contribution and stage buffers per member
+  // barrier state, second stage buffer per member
   int fgrid = 0;
   size_t fsmem = 0;
   GridBar *bar = nullptr;
-  std::vector<double *> C2, Vst2;
+  std::vector<double *> Vst2;
   std::vector<GP> gps;
   std::vector<BMember> bms;
   std::vector<void *> scratch;
@@ -2103,31 +2151,48 @@ int batch_fail(cgd_batch *b, cudaError_t e, const char *what)
     if (e_ != cudaSuccess) return batch_fail(b, e_, #call); \
   } while (0)
 
+// Levels of the single-member kernels' tiles.
+struct BatchTiles {
+  int hv1, p2;
+};
+template <int N>
+BatchTiles batch_tiles_n(bool mix)
+{
+  return {mix ? HV1Tile<N, float>::LT : HV1Tile<N, double>::LT, P2Cfg<N, 0, double>::LT};
+}
+BatchTiles batch_tiles(const cgd_batch *b)
+{
+  switch (b->N) {
+    case 2: return batch_tiles_n<2>(b->mix);
+    case 3: return batch_tiles_n<3>(b->mix);
+    case 4: return batch_tiles_n<4>(b->mix);
+    default: return batch_tiles_n<5>(b->mix);
+  }
+}
+
 // Work items of every kernel of a stage for every member, in one of three
 // orders: members one after the other, the largest member first, or the
 // members' items interleaved one by one.
-void batch_lists(const cgd_batch *b, int order, std::vector<WItem> out[BATCH_LISTS])
+void batch_lists(const cgd_batch *b, int order, std::vector<WItem> out[WL_N])
 {
   const int nm = (int)b->mem.size();
-  std::vector<std::vector<WItem>> per[BATCH_LISTS];
-  for (int k = 0; k < BATCH_LISTS; ++k) per[k].resize(nm);
-  const int DoF = b->N * b->N;
-  const int LT = 256 / DoF;
-  const int LTW = b->mix ? LT : (b->N == 5 ? HV1Tile<5, double>::LT : LT);   // list 5
-  const int LC = phase2_levels(b->N, cgd_batch::FORM_SPLIT), LCF = FUSED_P2_LEVELS;
+  std::vector<std::vector<WItem>> per[WL_N];
+  for (int k = 0; k < WL_N; ++k) per[k].resize(nm);
+  const BatchTiles T = batch_tiles(b);
   for (int m = 0; m < nm; ++m) {
     const cgd_handle *h = b->mem[m];
-    for (int IF = 0; IF < h->NF; ++IF)
-      for (int t = 0; t < (h->nz + LT - 1) / LT; ++t) per[0][m].push_back({m, t, IF});
-    const long long ncl = (long long)h->nz * h->NumG;
-    for (long long t = 0; t < (ncl + 255) / 256; ++t) per[1][m].push_back({m, (int)t, 0});
-    for (int IF = 0; IF < h->NF; ++IF)
-      for (int c = 0; c < 2 * ((h->nz + LC - 1) / LC); ++c) per[2][m].push_back({m, c, IF});
-    for (int c = 0; c < (h->NumG + COL_WARPS - 1) / COL_WARPS; ++c) per[3][m].push_back({m, c, 0});
-    for (int IF = 0; IF < h->NF; ++IF)
-      for (int c = 0; c < 2 * ((h->nz + LCF - 1) / LCF); ++c) per[4][m].push_back({m, c, IF});
-    for (int IF = 0; IF < h->NF; ++IF)
-      for (int t = 0; t < (h->nz + LTW - 1) / LTW; ++t) per[5][m].push_back({m, t, IF});
+    const bool flat = h->gp.flat != 0;
+    // x fastest: the tiles (and the two roles of phase 2) of one element
+    auto fill = [&](int list, int levels, int roles) {
+      for (int y = 0; y < h->NF; ++y)
+        for (int x = 0; x < roles * ((h->nz + levels - 1) / levels); ++x) per[list][m].push_back({m, x, y});
+    };
+    fill(flat ? WL_HV1F : WL_HV1, T.hv1, 1);
+    fill(flat ? WL_P2F : WL_P2, T.p2, 2);
+    fill(flat ? WL_P2AF : WL_P2A, P2_ALT_LEVELS, 2);
+    fill(WL_FHV1, 256 / (b->N * b->N), 1);
+    fill(WL_FP2, FUSED_P2_LEVELS, 2);
+    for (int c = 0; c < (h->NumG + COL_WARPS - 1) / COL_WARPS; ++c) per[WL_COL][m].push_back({m, c, 0});
   }
   std::vector<int> ord(nm);
   for (int m = 0; m < nm; ++m) ord[m] = m;
@@ -2135,7 +2200,7 @@ void batch_lists(const cgd_batch *b, int order, std::vector<WItem> out[BATCH_LIS
     std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) {
       return (long long)b->mem[a]->NF * b->mem[a]->nz > (long long)b->mem[c]->NF * b->mem[c]->nz;
     });
-  for (int k = 0; k < BATCH_LISTS; ++k) {
+  for (int k = 0; k < WL_N; ++k) {
     out[k].clear();
     if (order == 2) {
       size_t mx = 0;
@@ -2154,35 +2219,59 @@ void batch_enqueue_t(cgd_batch *b, WItem *const *w, bool p2alt)
 {
   using CF = P2Cfg<N, NT, R>;
   using CFA = P2Cfg<N, NT, R, P2_ALT_LEVELS>;
+  using HT = HV1Tile<N, R>;
+#ifdef CGD_FAST
+  using FF = P2Flat<N, NT, R>;
+  using FFA = P2Flat<N, NT, R, P2_ALT_LEVELS>;
+#endif
+  constexpr bool C32 = sizeof(R) == sizeof(float);
+  constexpr size_t hsmem = HV1Smem<N, NT, R, HT::LT>::BYTES;
   static std::atomic<unsigned long long> attr{0};
   const size_t csmem = (size_t)COL_WARPS * COL_ARR * b->nzmax * sizeof(double);
+  auto limit = [](auto f, size_t bytes) {
+    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
   if (first_on_device(attr)) {
-    cudaFuncSetAttribute(kb_phase2<N, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::SMEM);
-    cudaFuncSetAttribute(kb_hypervisc1w<N, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)HV1Smem<N, NT, R, HV1Tile<N, R>::LT>::BYTES);
-    if constexpr (N == 5)
-      cudaFuncSetAttribute(kb_phase2<N, NT, R, P2_ALT_LEVELS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)CFA::SMEM);
-    constexpr bool C32 = sizeof(R) == sizeof(float);
+    limit(kb_phase2<N, NT, R>, CF::SMEM);
+    limit(kb_hypervisc1<N, NT, R>, hsmem);
+    if constexpr (N == 5) limit(kb_phase2<N, NT, R, P2_ALT_LEVELS>, CFA::SMEM);
+#ifdef CGD_FAST
+    limit(kb_phase2_flat<N, NT, R>, FF::SMEM);
+    limit(kb_hypervisc1_flat<N, NT, R>, hsmem);
+    if constexpr (N == 5) limit(kb_phase2_flat<N, NT, R, P2_ALT_LEVELS>, FFA::SMEM);
+#endif
     for (auto f : {kb_column<0, C32>, kb_column<1, C32>, kb_column<2, C32>})
-      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, COL_WARPS * COL_ARR * 64 * (int)sizeof(double));
+      limit(f, COL_WARPS * COL_ARR * 64 * sizeof(double));
   }
-  kb_pressure<<<b->n[1], 256, 0, b->stream>>>(w[1], 0);
+  // (a list is empty when no member is of its kind)
+  const int *n = b->n;
   for (int stage = 0; stage < 3; ++stage) {
-    using HT = HV1Tile<N, R>;
-    kb_hypervisc1w<N, NT, R><<<b->n[5], HT::THREADS, HV1Smem<N, NT, R, HT::LT>::BYTES, b->stream>>>(w[5], stage);
-    kb_gather<sizeof(R) == sizeof(float)><<<b->n[1], 256, 0, b->stream>>>(w[1]);
+    if (n[WL_HV1]) kb_hypervisc1<N, NT, R><<<n[WL_HV1], HT::THREADS, hsmem, b->stream>>>(w[WL_HV1], stage);
+#ifdef CGD_FAST
+    if (n[WL_HV1F]) kb_hypervisc1_flat<N, NT, R><<<n[WL_HV1F], HT::THREADS, hsmem, b->stream>>>(w[WL_HV1F], stage);
+#endif
+    bool alt = false;
     if constexpr (N == 5) {
-      if (p2alt) kb_phase2<N, NT, R, P2_ALT_LEVELS><<<b->n[4], CFA::THREADS, CFA::SMEM, b->stream>>>(w[4], stage);
-      else kb_phase2<N, NT, R><<<b->n[2], CF::THREADS, CF::SMEM, b->stream>>>(w[2], stage);
-    } else {
-      kb_phase2<N, NT, R><<<b->n[2], CF::THREADS, CF::SMEM, b->stream>>>(w[2], stage);
+      if (p2alt) {
+        alt = true;
+        if (n[WL_P2A])
+          kb_phase2<N, NT, R, P2_ALT_LEVELS><<<n[WL_P2A], CFA::THREADS, CFA::SMEM, b->stream>>>(w[WL_P2A], stage);
+#ifdef CGD_FAST
+        if (n[WL_P2AF])
+          kb_phase2_flat<N, NT, R, P2_ALT_LEVELS>
+              <<<n[WL_P2AF], FFA::THREADS, FFA::SMEM, b->stream>>>(w[WL_P2AF], stage);
+#endif
+      }
     }
-    constexpr bool C32 = sizeof(R) == sizeof(float);
-    if (stage == 0) kb_column<0, C32><<<b->n[3], 32 * COL_WARPS, csmem, b->stream>>>(w[3]);
-    else if (stage == 1) kb_column<1, C32><<<b->n[3], 32 * COL_WARPS, csmem, b->stream>>>(w[3]);
-    else kb_column<2, C32><<<b->n[3], 32 * COL_WARPS, csmem, b->stream>>>(w[3]);
-    if (stage < 2) kb_pressure<<<b->n[1], 256, 0, b->stream>>>(w[1], 1);
+    if (!alt) {
+      if (n[WL_P2]) kb_phase2<N, NT, R><<<n[WL_P2], CF::THREADS, CF::SMEM, b->stream>>>(w[WL_P2], stage);
+#ifdef CGD_FAST
+      if (n[WL_P2F]) kb_phase2_flat<N, NT, R><<<n[WL_P2F], FF::THREADS, FF::SMEM, b->stream>>>(w[WL_P2F], stage);
+#endif
+    }
+    if (stage == 0) kb_column<0, C32><<<n[WL_COL], 32 * COL_WARPS, csmem, b->stream>>>(w[WL_COL]);
+    else if (stage == 1) kb_column<1, C32><<<n[WL_COL], 32 * COL_WARPS, csmem, b->stream>>>(w[WL_COL]);
+    else kb_column<2, C32><<<n[WL_COL], 32 * COL_WARPS, csmem, b->stream>>>(w[WL_COL]);
   }
 }
 
@@ -2216,7 +2305,7 @@ template <int NT, typename R>
 cudaError_t batch_enqueue_fused_t(cgd_batch *b, WItem *const *w)
 {
   FusedArgs fa{};
-  for (int k = 0; k < 5; ++k) {
+  for (int k = 0; k < WL_N; ++k) {
     fa.w[k] = w[k];
     fa.n[k] = b->n[k];
   }
@@ -2260,6 +2349,7 @@ cudaError_t fused_setup_t(cgd_batch *b)
   using CF = P2Cfg<5, NT, R, FUSED_P2_LEVELS>;
   const size_t csm = (size_t)COL_WARPS * COL_ARR * b->nzmax * sizeof(double);
   b->fsmem = std::max(std::max(CF::SMEM, csm), HV1Smem<5, NT, R>::BYTES);
+  static_assert(P2Flat<5, NT, R, FUSED_P2_LEVELS>::SMEM <= CF::SMEM, "the flat phase 2 needs no more");
   cudaError_t e = cudaFuncSetAttribute(kb_stage<5, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->fsmem);
   if (e != cudaSuccess) return e;
   int per_sm = 0, sms = 0;
@@ -2415,22 +2505,20 @@ int cgd_batch_create(cgd_handle *const *members, int32_t nmembers, int32_t flags
       for (int m = 0; m < nmembers && e == cudaSuccess; ++m) {
         const cgd_handle *h = members[m];
         const size_t S = (size_t)h->nz * h->NumG;
-        const size_t ENL = (size_t)h->N * h->N * h->nz * h->NF;
-        void *c2 = nullptr, *v2 = nullptr;
-        e = cudaMalloc(&c2, ENL * (h->NV + 1) * sizeof(double));
-        b->C2.push_back(static_cast<double *>(c2));
-        if (e == cudaSuccess) e = cudaMalloc(&v2, S * h->NV * sizeof(double));
+        void *v2 = nullptr;
+        e = cudaMalloc(&v2, S * h->NV * sizeof(double));
         b->Vst2.push_back(static_cast<double *>(v2));
       }
       if (e != cudaSuccess) { rc = batch_fail(b, e, "cgd_batch_create fused buffers"); break; }
     }
     const int nord = b->autotune ? cgd_batch::NORD : 1;
     for (int o = 0; o < nord && !rc; ++o) {
-      std::vector<WItem> lists[BATCH_LISTS];
+      std::vector<WItem> lists[WL_N];
       batch_lists(b, o, lists);
-      for (int k = 0; k < BATCH_LISTS; ++k) {
+      for (int k = 0; k < WL_N; ++k) {
         b->n[k] = (int)lists[k].size();
         void *p = nullptr;
+        if (lists[k].empty()) continue;
         e = cudaMalloc(&p, lists[k].size() * sizeof(WItem));
         if (e == cudaSuccess)
           e = cudaMemcpy(p, lists[k].data(), lists[k].size() * sizeof(WItem), cudaMemcpyHostToDevice);
@@ -2456,10 +2544,9 @@ void cgd_batch_destroy(cgd_batch *b)
     if (b->graph[c]) cudaGraphDestroy(b->graph[c]);
   }
   for (int o = 0; o < cgd_batch::NORD; ++o)
-    for (int k = 0; k < BATCH_LISTS; ++k)
+    for (int k = 0; k < WL_N; ++k)
       if (b->w[o][k]) cudaFree(b->w[o][k]);
   for (void *p : b->scratch) cudaFree(p);
-  for (double *p : b->C2) if (p) cudaFree(p);
   for (double *p : b->Vst2) if (p) cudaFree(p);
   if (b->bar) cudaFree(b->bar);
   if (b->order_ev) cudaEventDestroy(b->order_ev);
@@ -2493,8 +2580,8 @@ int cgd_batch_step(cgd_batch *b, double *const *U, const double *dt, int32_t nst
   auto set_members = [&](double *const *state) {
     for (int m = 0; m < nm; ++m) {
       const cgd_handle *h = b->mem[m];
-      b->bms[m] = BMember{state[m], h->Vst, h->k1, h->k2, h->C, h->T1, h->jbg, h->pres, h->pres_st, dt[m],
-                          b->C2.empty() ? nullptr : b->C2[m], b->Vst2.empty() ? nullptr : b->Vst2[m]};
+      b->bms[m] = BMember{state[m], h->Vst, h->k1, h->k2, h->C1, h->C, h->jbg, h->pres, dt[m],
+                          b->Vst2.empty() ? nullptr : b->Vst2[m]};
     }
   };
   // the members form's graph for the given states and time steps (captured

@@ -6,18 +6,17 @@
 // A work item is (member, block x, block y) of the member's own launch grid;
 // the kernel bodies are the single-member ones, given the member's
 // parameters from constant memory.  One ensemble step is one CUDA graph of
-// 15 launches, whatever the number of members.
+// 9 launches, whatever the number of members.
 //
-// The fused form (kb_stage, p = 4) runs a whole stage - pressure, phase 1,
-// its DSS, phase 2, the column solve and update, the next stage's pressure -
-// as one persistent cooperative launch whose CTAs walk the same work lists,
+// The fused form (kb_stage, p = 4) runs a whole stage - phase 1 with the
+// pressure, phase 2, the column solve and update - as one persistent cooperative launch whose CTAs walk the same work lists,
 // with a grid barrier between the parts: one ensemble step is three
 // launches.  Within one launch no array is read, rewritten and read again
-// (phase 2 writes a second contribution buffer C2, the stage-3 state goes to
+// (the phases write contribution buffers of their own, the stage-3 state goes to
 // a second stage buffer Vst2), so no CTA can read a line that an earlier part
 // of the same launch left in its caches before another CTA rewrote it.
 #pragma once
-#include "cgd_phase2.cuh"
+#include "cgd_flat.cuh"
 
 namespace cgd {
 
@@ -25,10 +24,10 @@ constexpr int BMAX = 64;   // members of one ensemble
 
 struct BMember {
   double *U;                     // the member's state (device), updated in place
-  double *Vst, *k1, *k2, *C, *T1, *jbg;
-  double *P0, *Pst;              // pressure of the state and of the stage state
+  double *Vst, *k1, *k2, *C1, *C, *jbg;
+  double *pres;                  // pressure of the stage state
   double dt;
-  double *C2, *Vst2;             // fused form only: phase-2 contributions, stage-3 state
+  double *Vst2;                  // fused form only: stage-3 state
 };
 
 struct WItem {
@@ -39,33 +38,28 @@ __constant__ GP c_bgp[BMAX];
 __constant__ BMember c_bm[BMAX];
 __constant__ RK c_brk;
 
-// Phase 1 of the split form, with the single-member kernel's level tile
-// (HV1Tile) and its dynamic shared memory.
+// Phase 1 and phase 2 of the split form, in the single-member kernels' tiles:
+// the members of a general grid, and those of a flat product grid.
 template <int N, int NT, typename R>
 __global__ void __launch_bounds__(HV1Tile<N, R>::THREADS, HV1Tile<N, R>::MINB)
-    kb_hypervisc1w(const WItem *__restrict__ w, const int stage)
+    kb_hypervisc1(const WItem *__restrict__ w, const int stage)
 {
   extern __shared__ __align__(16) unsigned char hvb_dyn[];
   const WItem it = w[blockIdx.x];
   const BMember &B = c_bm[it.m];
-  hypervisc1_body<N, NT, R, HV1Tile<N, R>::LT>(c_bgp[it.m], stage == 0 ? B.U : B.Vst, B.C, it.x, it.y,
+  hypervisc1_body<N, NT, R, HV1Tile<N, R>::LT>(c_bgp[it.m], stage == 0 ? B.U : B.Vst, B.C1, B.pres, it.x, it.y,
                                                reinterpret_cast<R *>(hvb_dyn));
 }
 
-__global__ void __launch_bounds__(256) kb_pressure(const WItem *__restrict__ w, const int stage_state)
+template <int N, int NT, typename R>
+__global__ void __launch_bounds__(HV1Tile<N, R>::THREADS, HV1Tile<N, R>::MINB)
+    kb_hypervisc1_flat(const WItem *__restrict__ w, const int stage)
 {
+  extern __shared__ __align__(16) unsigned char hvb_dyn[];
   const WItem it = w[blockIdx.x];
   const BMember &B = c_bm[it.m];
-  pressure_body(c_bgp[it.m], stage_state ? B.Vst : B.U, stage_state ? B.Pst : B.P0,
-                (long long)it.x * blockDim.x + threadIdx.x);
-}
-
-template <bool C32>
-__global__ void __launch_bounds__(256) kb_gather(const WItem *__restrict__ w)
-{
-  const WItem it = w[blockIdx.x];
-  const BMember &B = c_bm[it.m];
-  gather_body<false, true, C32>(c_bgp[it.m], B.C, B.T1, (long long)it.x * blockDim.x + threadIdx.x);
+  hypervisc1_flat<N, NT, R, HV1Tile<N, R>::LT>(c_bgp[it.m], stage == 0 ? B.U : B.Vst, B.C1, B.pres, it.x, it.y,
+                                               reinterpret_cast<R *>(hvb_dyn));
 }
 
 // LT: levels per phase-2 CTA
@@ -75,7 +69,16 @@ __global__ void __launch_bounds__(P2Cfg<N, NT, R, LT>::THREADS, P2Cfg<N, NT, R, 
 {
   const WItem it = w[blockIdx.x];
   const BMember &B = c_bm[it.m];
-  phase2_body<N, NT, R, LT>(c_bgp[it.m], stage == 0 ? B.U : B.Vst, stage == 0 ? B.P0 : B.Pst, B.T1, B.C, it.x, it.y);
+  phase2_body<N, NT, R, LT>(c_bgp[it.m], stage == 0 ? B.U : B.Vst, B.pres, B.C1, B.C, it.x, it.y);
+}
+
+template <int N, int NT, typename R, int LT = p2_levels<N>()>
+__global__ void __launch_bounds__(P2Flat<N, NT, R, LT>::THREADS, P2Flat<N, NT, R, LT>::MINB)
+    kb_phase2_flat(const WItem *__restrict__ w, const int stage)
+{
+  const WItem it = w[blockIdx.x];
+  const BMember &B = c_bm[it.m];
+  phase2_flat<N, NT, R, LT>(c_bgp[it.m], stage == 0 ? B.U : B.Vst, B.pres, B.C1, B.C, it.x, it.y);
 }
 
 template <int MODE, bool C32>
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(32 * COL_WARPS, 4) kb_column(const WItem *__re
   a.fac = B.dt * c_brk.gamma;
   a.rk = c_brk;
   a.Vs = MODE == 0 ? B.U : B.Vst;
-  a.ps = MODE == 0 ? B.P0 : B.Pst;
+  a.ps = B.pres;
   if (MODE == 0) { a.kout = B.k1; a.Vout = B.Vst; }
   else if (MODE == 1) { a.kout = B.k2; a.Vout = B.Vst; }
   else { a.kout = nullptr; a.Vout = B.U; }
@@ -180,16 +183,18 @@ __global__ void __launch_bounds__(256) k_barrier_probe(GridBar *gb, unsigned lon
   }
 }
 
-// work lists of the fused kernel: 0 phase-1 tiles, 1 blocks of 256
-// column-levels (DSS gather, pressure), 3 blocks of COL_WARPS columns, 4
-// phase-2 items of FUSED_P2_LEVELS levels (200 of the 256 threads)
-constexpr int FUSED_P2_LEVELS = 8;
-// the split form's alternative phase-2 CTA for p = 4 (autotuner), on the fused form's list
+// Work lists of an ensemble (WItem x, y of the member's launch grid): phase-1
+// tiles and phase-2 items of the general members and of the flat ones, the
+// phase-2 items of 8-level CTAs (p = 4: the split form's alternative), the
+// column blocks, and the fused kernel's phase-1 and phase-2 items (all members;
+// P.flat says of which kind).
+enum { WL_HV1 = 0, WL_HV1F, WL_P2, WL_P2F, WL_P2A, WL_P2AF, WL_COL, WL_FHV1, WL_FP2, WL_N };
 constexpr int P2_ALT_LEVELS = 8;
-static_assert(P2_ALT_LEVELS == FUSED_P2_LEVELS, "work list 4 serves both");
+// the fused kernel's 256-thread CTAs: phase 2 takes 8 levels (200 threads)
+constexpr int FUSED_P2_LEVELS = 8;
 struct FusedArgs {
-  const WItem *w[5];
-  int n[5];
+  const WItem *w[WL_N];
+  int n[WL_N];
   GridBar *bar;
 };
 
@@ -207,44 +212,42 @@ __global__ void __launch_bounds__(256, 2) kb_stage(const FusedArgs A, const int 
   static_assert(P2Cfg<N, NT, R, FUSED_P2_LEVELS>::THREADS <= 256, "phase-2 items of 256 threads");
   static_assert(32 * COL_WARPS == 256, "column blocks of 256 threads");
   extern __shared__ double fsm[];   // each part's shared arrays in turn (phase 1, phase 2, column)
-  if (stage == 0) {   // pressure of the step's state
-    for (int i = blockIdx.x; i < A.n[1]; i += gridDim.x) {
-      const WItem it = A.w[1][i];
-      const BMember &B = c_bm[it.m];
-      pressure_body(c_bgp[it.m], B.U, B.P0, (long long)it.x * 256 + threadIdx.x);
-    }
-    if (!grid_sync(A.bar)) return;
-  }
-  // phase 1 of the hyperviscosity -> C
-  for (int i = blockIdx.x; i < A.n[0]; i += gridDim.x) {
-    const WItem it = A.w[0][i];
+  // phase 1 of the hyperviscosity and the pressure -> C1, pres
+  for (int i = blockIdx.x; i < A.n[WL_FHV1]; i += gridDim.x) {
+    const WItem it = A.w[WL_FHV1][i];
     const BMember &B = c_bm[it.m];
-    hypervisc1_body<N, NT, R>(c_bgp[it.m], fused_stage_state(B, stage), B.C, it.x, it.y, reinterpret_cast<R *>(fsm));
+    R *const s = reinterpret_cast<R *>(fsm);
+#ifdef CGD_FAST
+    if (c_bgp[it.m].flat)
+      hypervisc1_flat<N, NT, R, 256 / (N * N)>(c_bgp[it.m], fused_stage_state(B, stage), B.C1, B.pres, it.x, it.y,
+                                               s);
+    else
+#endif
+      hypervisc1_body<N, NT, R>(c_bgp[it.m], fused_stage_state(B, stage), B.C1, B.pres, it.x, it.y, s);
     __syncthreads();   // the next item reuses the shared arrays
   }
   if (!grid_sync(A.bar)) return;
-  // its DSS -> T1
-  for (int i = blockIdx.x; i < A.n[1]; i += gridDim.x) {
-    const WItem it = A.w[1][i];
+  // phase 2 -> C
+  for (int i = blockIdx.x; i < A.n[WL_FP2]; i += gridDim.x) {
+    const WItem it = A.w[WL_FP2][i];
     const BMember &B = c_bm[it.m];
-    gather_body<false, true, C32>(c_bgp[it.m], B.C, B.T1, (long long)it.x * 256 + threadIdx.x);
-  }
-  if (!grid_sync(A.bar)) return;
-  // phase 2 -> C2
-  for (int i = blockIdx.x; i < A.n[4]; i += gridDim.x) {
-    const WItem it = A.w[4][i];
-    const BMember &B = c_bm[it.m];
-    phase2_body<N, NT, R, FUSED_P2_LEVELS, 256>(c_bgp[it.m], fused_stage_state(B, stage),
-                                                stage == 0 ? B.P0 : B.Pst, B.T1, B.C2, it.x, it.y);
+#ifdef CGD_FAST
+    if (c_bgp[it.m].flat)
+      phase2_flat<N, NT, R, FUSED_P2_LEVELS, 256>(c_bgp[it.m], fused_stage_state(B, stage), B.pres, B.C1, B.C, it.x,
+                                                  it.y);
+    else
+#endif
+      phase2_body<N, NT, R, FUSED_P2_LEVELS, 256>(c_bgp[it.m], fused_stage_state(B, stage), B.pres, B.C1, B.C, it.x,
+                                                  it.y);
     __syncthreads();
   }
   if (!grid_sync(A.bar)) return;
   // owner gather of phase 2, Jacobian, Schur solve, stage update
-  for (int i = blockIdx.x; i < A.n[3]; i += gridDim.x) {
-    const WItem it = A.w[3][i];
+  for (int i = blockIdx.x; i < A.n[WL_COL]; i += gridDim.x) {
+    const WItem it = A.w[WL_COL][i];
     const BMember &B = c_bm[it.m];
     ColArgs a;
-    a.C = B.C2;
+    a.C = B.C;
     a.Vn = B.U;
     a.k1 = B.k1;
     a.k2 = B.k2;
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(256, 2) kb_stage(const FusedArgs A, const int 
     a.fac = B.dt * c_brk.gamma;
     a.rk = c_brk;
     a.Vs = fused_stage_state(B, stage);
-    a.ps = stage == 0 ? B.P0 : B.Pst;
+    a.ps = B.pres;
     if (stage == 0) {
       a.kout = B.k1; a.Vout = B.Vst;
       column_body<0, C32>(c_bgp[it.m], a, it.x);
@@ -267,14 +270,6 @@ __global__ void __launch_bounds__(256, 2) kb_stage(const FusedArgs A, const int 
       column_body<2, C32>(c_bgp[it.m], a, it.x);
     }
     __syncthreads();
-  }
-  if (stage == 2) return;
-  if (!grid_sync(A.bar)) return;
-  // pressure of the next stage state
-  for (int i = blockIdx.x; i < A.n[1]; i += gridDim.x) {
-    const WItem it = A.w[1][i];
-    const BMember &B = c_bm[it.m];
-    pressure_body(c_bgp[it.m], stage == 0 ? B.Vst : B.Vst2, B.Pst, (long long)it.x * 256 + threadIdx.x);
   }
 }
 

@@ -25,7 +25,13 @@
 // (k_flat_check, FLAT_TOL); any other grid, and the exact build, run the
 // general kernels (hypervisc1_body, phase2_body).
 //
-// Same tiles, roles and planes as cgd_phase2.cuh.
+// Same tiles, roles and planes as cgd_phase2.cuh.  nPanel 30, p 4, nz 45, two
+// tracers: phase 1 0.310 -> 0.238 ms (91 % of the L1/shared pipe's peak), phase
+// 2 1.224 -> 0.749 ms (67 % of it, 26 warps an SM waiting for loads and
+// barriers); before the pressure (phase 1, 0.027 ms) and the cache sums (phase
+// 2, 0.07 ms) came in from kernels of 0.041 and 0.115 ms.  Tried: a thread per row
+// of nodes with the x sums in registers, half the shared loads but 10 to 15
+// warps an SM: 1.29 ms.
 #pragma once
 #include "cgd_phase2.cuh"
 
@@ -41,104 +47,84 @@ __device__ __forceinline__ double ratio_of(double n, double d, double r)
   return fma(fma(-q, d, n), r, q);
 }
 
-// The factors, each the mean over the levels (z: over nodes) of what the
-// arrays hold, so that a factor is nearer to the arrays' common value than any
-// one rounded entry.
-// z(l) over z(0): the sums of J over up to FLAT_NODES element nodes; one CTA
-// per level.  Also 1/z.
-constexpr int FLAT_NODES = 8192;
-__global__ void __launch_bounds__(256) k_flat_z(const GP P, double *__restrict__ zl)
+// The layers' table zl: z from the nodes of the first element (their mean J, as
+// cgd_set_layers documents it), or the caller's zin; 1/z, the RecU4
+// coefficients and the slope residue.  One CTA of 64 threads.
+__global__ void __launch_bounds__(64) k_flat_layers(const GP P, const double *__restrict__ zin,
+                                                    double *__restrict__ zl)
 {
-  __shared__ double s0[256], s1[256];
-  const int l = blockIdx.x, nz = P.nz;
-  const long long n = (long long)P.NF * P.DoF;
-  const long long every = n > FLAT_NODES ? n / FLAT_NODES : 1;
-  double a = 0.0, b = 0.0;
-  for (long long i = threadIdx.x * every; i < n; i += 256 * every) {
-    const int IF = (int)(i / P.DoF), ID = (int)(i - (long long)IF * P.DoF);
-    const double *m = P.met + (((size_t)IF * NCOMP + C_J0) * P.DoF + ID) * nz;
-    a += m[l];
-    b += m[0];
-  }
-  s0[threadIdx.x] = a;
-  s1[threadIdx.x] = b;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      s0[threadIdx.x] += s0[threadIdx.x + w];
-      s1[threadIdx.x] += s1[threadIdx.x + w];
+  __shared__ double zs[64];
+  const int l = threadIdx.x, nz = P.nz, DoF = P.DoF, N = P.N;
+  const size_t cs = (size_t)DoF * nz;
+  const double *me = P.met;   // element 0
+  if (l < nz) {
+    double a = 0.0, b = 0.0;
+    for (int ID = 0; ID < DoF; ++ID) {
+      a += me[C_J0 * cs + (size_t)ID * nz + l];
+      b += me[C_J0 * cs + (size_t)ID * nz];
     }
-    __syncthreads();
+    zs[l] = zin ? zin[l] : a / b;
   }
-  if (threadIdx.x == 0) {
-    const double z = s0[0] / s1[0];
-    zl[l] = z;
-    zl[nz + l] = 1.0 / z;
+  __syncthreads();
+  if (l >= nz) return;
+  zl[l] = zs[l];
+  zl[nz + l] = 1.0 / zs[l];
+  double rk[4] = {0.0, 0.0, 0.0, 0.0};
+  if (l < nz - 1) {   // RecU4 (OperatorKernel.jl:1044-1059) with J = hJ z
+    const double LL = zs[l > 0 ? l - 1 : 0], L = zs[l], R = zs[l + 1], RR = zs[l + 2 < nz ? l + 2 : nz - 1];
+    rk[0] = (L / (L + R)) * ((LL + L) / (LL + L + R));
+    rk[1] = (L / (LL + L)) * (R / (LL + L + R));
+    rk[2] = (R / (R + L)) * ((RR + R) / (L + R + RR));
+    rk[3] = (R / (RR + R)) * (L / (L + R + RR));
+  }
+  for (int c = 0; c < 4; ++c) zl[(2 + c) * nz + l] = rk[c];
+  // slope residue: dXdxI(3,1) = -(h11 f(I) + h21 f(J)), (3,2) = -(h12 f(I) +
+  // h22 f(J)) with f(I, level, node) = sum_k DS[I,k] height, the same in every
+  // element; from the nodes (I, 0).  Kept: the sum over the two nodes of a
+  // layer and half their difference over z, in single precision (1e-23 of d33
+  // off, and the same digits whichever element they come from)
+  for (int I = 0; I < N; ++I) {
+    const double *m = me + (size_t)I * nz + l;
+    const double h11 = m[C_D11_0 * cs], h12 = m[C_D12_0 * cs], h21 = m[C_D21_0 * cs], h22 = m[C_D22_0 * cs];
+    const double rd = zs[l] / (h11 * h22 - h12 * h21);
+    double f[2];
+    for (int k = 0; k < 2; ++k) f[k] = (h21 * m[(C_D32_0 + k) * cs] - h22 * m[(C_D31_0 + k) * cs]) * rd;
+    zl[(size_t)(6 + I) * nz + l] = (float)(f[0] + f[1]);
+    zl[(size_t)(6 + N + I) * nz + l] = (float)(0.5 * (f[1] - f[0]) / zs[l]);
   }
 }
 
-// The element nodes' horizontal factors, the columns' 1 / m and (thread 0) the
-// interfaces' RecU4 coefficients; one thread per element node, then per column.
-__global__ void __launch_bounds__(256) k_flat_factors(const GP P, double *__restrict__ hm, double *__restrict__ zl,
-                                                      double *__restrict__ rmg)
+// The element nodes' factors, each the mean over the levels of what the arrays
+// hold, nearer to their common value than any one rounded entry.  One CTA of
+// 32 threads per element.
+__global__ void __launch_bounds__(32) k_flat_factors(const GP P, double *__restrict__ hm)
 {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int nz = P.nz, DoF = P.DoF;
+  const int IF = blockIdx.x, t = threadIdx.x, nz = P.nz, DoF = P.DoF;
+  if (t >= DoF) return;
   const size_t cs = (size_t)DoF * nz;
+  const double *m = P.met + (size_t)IF * NCOMP * cs + (size_t)t * nz;
   double sz = 0.0;
-  for (int l = 0; l < nz; ++l) sz += zl[l];
-  if (t == 0) {
-    for (int l = 0; l < nz - 1; ++l) {   // RecU4 (OperatorKernel.jl:1044-1059) with J = hJ z
-      const double LL = zl[l > 0 ? l - 1 : 0], L = zl[l], R = zl[l + 1], RR = zl[l + 2 < nz ? l + 2 : nz - 1];
-      zl[2 * nz + l] = (L / (L + R)) * ((LL + L) / (LL + L + R));
-      zl[3 * nz + l] = (L / (LL + L)) * (R / (LL + L + R));
-      zl[4 * nz + l] = (R / (R + L)) * ((RR + R) / (L + R + RR));
-      zl[5 * nz + l] = (R / (RR + R)) * (L / (L + R + RR));
-    }
-    for (int c = 2; c < 6; ++c) zl[c * nz + nz - 1] = 0.0;
-  }
-  const long long nn = (long long)P.NF * DoF;
-  if (t < (long long)P.N * nz) {
-    // slope residue: dXdxI(3,1) = -(h11 f(I) + h21 f(J)), (3,2) = -(h12 f(I) +
-    // h22 f(J)) with f(I, level, node) = sum_k DS[I,k] height, the same in every
-    // element; from the nodes (I, 0) of the first one.  Kept: the sum over the
-    // two nodes of a layer and half their difference over z
-    const int I = (int)(t / nz), l = (int)(t - (long long)I * nz);
-    const double *m = P.met + (size_t)I * nz + l;
-    const double h11 = m[C_D11_0 * cs], h12 = m[C_D12_0 * cs], h21 = m[C_D21_0 * cs], h22 = m[C_D22_0 * cs];
-    const double rd = zl[l] / (h11 * h22 - h12 * h21);
-    double f[2];
-    for (int k = 0; k < 2; ++k) f[k] = (h21 * m[(C_D32_0 + k) * cs] - h22 * m[(C_D31_0 + k) * cs]) * rd;
-    zl[(size_t)(6 + I) * nz + l] = f[0] + f[1];
-    zl[(size_t)(6 + P.N + I) * nz + l] = 0.5 * (f[1] - f[0]) / zl[l];
-  }
-  if (t < nn) {
-    const int IF = (int)(t / DoF), ID = (int)(t - (long long)IF * DoF);
-    const double *m = P.met + ((size_t)IF * NCOMP * DoF + ID) * nz;
-    auto mean = [&](int c) {   // of both nodes of the layers, over z
-      double a = 0.0;
-      for (int l = 0; l < nz; ++l) a += m[c * cs + l] + m[(c + 1) * cs + l];
-      return 0.5 * a / sz;
-    };
-    double *o = hm + (size_t)IF * H_N * DoF + ID;
-    for (int c = 0; c < 4; ++c) o[(H_11 + c) * DoF] = mean(C_D11_0 + 2 * c);
-    const double hJ = mean(C_J0);
-    o[H_J * DoF] = hJ;
-    o[H_RJ * DoF] = 1.0 / hJ;
-    o[H_33 * DoF] = m[C_D33_0 * cs];
-    o[H_FC * DoF] = m[C_FCOR * cs];
-    return;
-  }
-  const long long g = t - nn;
-  if (g >= P.NumG) return;
+  for (int l = 0; l < nz; ++l) sz += P.zl[l];
+  auto mean = [&](int c) {   // of both nodes of the layers, over z
+    double a = 0.0;
+    for (int l = 0; l < nz; ++l) a += m[c * cs + l] + m[(c + 1) * cs + l];
+    return 0.5 * a / sz;
+  };
+  double *o = hm + (size_t)IF * H_N * DoF + t;
+  for (int c = 0; c < 4; ++c) o[(H_11 + c) * DoF] = mean(C_D11_0 + 2 * c);
+  const double hJ = mean(C_J0);
+  o[H_J * DoF] = hJ;
+  o[H_RJ * DoF] = 1.0 / hJ;
+  o[H_33 * DoF] = m[C_D33_0 * cs];
+  o[H_FC * DoF] = m[C_FCOR * cs];
+  const size_t g = P.glob[IF * DoF + t];
   double a = 0.0;
-  for (int l = 0; l < nz; ++l) a += P.M[l + (size_t)nz * g] + P.M[l + (size_t)nz * (g + P.NumG)];
-  rmg[g] = 2.0 * sz / a;
+  for (int l = 0; l < nz; ++l) a += P.M[l + nz * g] + P.M[l + nz * (g + P.NumG)];
+  o[H_RM * DoF] = 2.0 * sz / a;
 }
 
 // Sets *bad unless every entry of the metric and the lumped mass is its
-// product of factors to FLAT_TOL.  One thread per element node and level, then
-// one per column and level.
+// product of factors to FLAT_TOL.  One thread per element node and level.
 __global__ void __launch_bounds__(256) k_flat_check(const GP P, double Omega2, int *__restrict__ bad)
 {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -146,13 +132,15 @@ __global__ void __launch_bounds__(256) k_flat_check(const GP P, double Omega2, i
   const size_t cs = (size_t)DoF * nz;
   const long long ne = (long long)P.NF * DoF * nz;
   auto differ = [](double a, double b, double scale) { return !(fabs(a - b) <= FLAT_TOL * scale); };
-  if (t < ne) {
+  if (t >= ne) return;
+  {
     const int l = (int)(t % nz);
     const long long n = t / nz;
     const int ID = (int)(n % DoF), IF = (int)(n / DoF);
     const double *m = P.met + ((size_t)IF * NCOMP * DoF + ID) * nz + l;
     const double *h = P.hm + (size_t)IF * H_N * DoF + ID;
-    const double z = P.zl[l], h33 = h[H_33 * DoF], hJ = h[H_J * DoF];
+    const double *zt = P.zl;
+    const double z = zt[l], h33 = h[H_33 * DoF], hJ = h[H_J * DoF];
     double mx = 0.0;
     for (int c = 0; c < 4; ++c) mx = fmax(mx, fabs(h[(H_11 + c) * DoF]));
     bool b = !(h33 > 0.0) || !(hJ > 0.0) || !(z > 0.0);
@@ -163,7 +151,7 @@ __global__ void __launch_bounds__(256) k_flat_check(const GP P, double Omega2, i
       b = b || differ(m[(C_D31_0 + k) * cs], 0.0, h33) || differ(m[(C_D32_0 + k) * cs], 0.0, h33);
     }
     // the slope residue against its factors: to a hundredth of a rounding of d33
-    const double *sl = P.zl + (size_t)6 * nz + l;
+    const double *sl = zt + (size_t)6 * nz + l;
     const int I = ID % P.N, J = ID / P.N;
     const double sI = sl[I * nz], sJ = sl[J * nz];
     const double dI = 2.0 * z * sl[(P.N + I) * nz], dJ = 2.0 * z * sl[(P.N + J) * nz];
@@ -175,14 +163,12 @@ __global__ void __launch_bounds__(256) k_flat_check(const GP P, double Omega2, i
     }
     b = b || differ(m[C_FCOR * cs], h[H_FC * DoF], Omega2);
     if (l < nz - 1)
-      for (int c = 0; c < 4; ++c) b = b || differ(m[(C_RK0 + c) * cs], P.zl[(2 + c) * nz + l], 1.0);
+      for (int c = 0; c < 4; ++c) b = b || differ(m[(C_RK0 + c) * cs], zt[(2 + c) * nz + l], 1.0);
+    const size_t o = l + (size_t)nz * P.glob[IF * DoF + ID];
+    const double rm = h[H_RM * DoF], x0 = P.M[o] * rm, x1 = P.M[o + (size_t)nz * P.NumG] * rm;
+    b = b || !(rm > 0.0) || differ(x0, z, z) || differ(x1, z, z);
     if (b) *bad = 1;
-    return;
   }
-  const long long s = t - ne, S = (long long)nz * P.NumG;
-  if (s >= S) return;
-  const double rm = P.rmg[s / nz], x0 = P.M[s] * rm, x1 = P.M[s + S] * rm, z = P.zl[s % nz];
-  if (!(rm > 0.0) || differ(x0, z, z) || differ(x1, z, z)) *bad = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -190,7 +176,7 @@ __global__ void __launch_bounds__(256) k_flat_check(const GP P, double Omega2, i
 // ---------------------------------------------------------------------------
 template <int N, int NT, typename R, int LT>
 __device__ __forceinline__ void hypervisc1_flat(const GP &P, const double *__restrict__ U, double *__restrict__ C,
-                                                const int tile, const int IF, R *sbuf)
+                                                double *__restrict__ Pr, const int tile, const int IF, R *sbuf)
 {
   constexpr bool MIX = sizeof(R) == sizeof(float);
   using CT = typename std::conditional<MIX, float, double>::type;
@@ -210,7 +196,7 @@ __device__ __forceinline__ void hypervisc1_flat(const GP &P, const double *__res
     const double *h = P.hm + (size_t)IF * H_N * DoF + ID;
     h11 = (R)h[H_11 * DoF]; h12 = (R)h[H_12 * DoF]; h21 = (R)h[H_21 * DoF]; h22 = (R)h[H_22 * DoF];
     rJ = (R)h[H_RJ * DoF];
-    rm = (R)P.rmg[g];
+    rm = (R)h[H_RM * DoF];
     const double *Ug = U + l + (size_t)nz * g;
     const size_t fs = (size_t)nz * P.NumG;
     const R u = (R)Ug[1 * fs], v = (R)Ug[2 * fs];
@@ -222,6 +208,7 @@ __device__ __forceinline__ void hypervisc1_flat(const GP &P, const double *__res
     s[4][si] = (R)(ratio_of(Ug[4 * fs], rho, rr) - (MIX ? P.thref[l] : 0.0));
 #pragma unroll
     for (int q = 0; q < NT; ++q) s[9 + 3 * q][si] = (R)ratio_of(Ug[(5 + q) * fs], rho, rr);
+    stage_pressure(P, Pr, IF * DoF + ID, g, l, Ug[4 * fs]);
   }
   __syncthreads();
   if (act) {
@@ -313,7 +300,7 @@ struct P2Flat {
 
 template <int N, int NT, typename R, int LT, int TH>
 __device__ __forceinline__ void phase2_scalars_flat(const GP &P, const double *__restrict__ U,
-                                                    const double *__restrict__ T1, double *__restrict__ C,
+                                                    const double *__restrict__ C1, double *__restrict__ C,
                                                     const int L0, const int IF, double *sm)
 {
   using CF = P2Flat<N, NT, R, LT>;
@@ -344,16 +331,17 @@ __device__ __forceinline__ void phase2_scalars_flat(const GP &P, const double *_
   if (act) {
     const int g = P.glob[IF * DoF + ID];
     const double *Ug = U + (size_t)nz * g + l;
-    const CT *T = reinterpret_cast<const CT *>(T1) + (size_t)nz * g + l;
+    R ca[NS];
+    cache_sums<MIX, 4, NS>(P, C1, IF * DoF + ID, l, ca);
     rho = Ug[0];
     const double u = Ug[fs], v = Ug[2 * fs];
     F0 = Ug[3 * fs] * (rho + (l < nz - 1 ? Ug[1] : 0.0));   // mass flux of interface l over d33
     const double a11 = hn[H_11 * DoF], a12 = hn[H_12 * DoF], a21 = hn[H_21 * DoF], a22 = hn[H_22 * DoF];
-    rm = P.rmg[g];
+    rm = hn[H_RM * DoF];
     const double rr = 1.0 / rho;
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
-      sc[q * PL + si] = (R)T[(4 + q) * fs];
+      sc[q * PL + si] = ca[q];
       const double c = ratio_of(Ug[(4 + q) * fs], rho, rr);
       cth[(q * CR + lvl + 2) * RS + ID] = c;
       if (MIX) sq[q * PL + si] = (R)c;
@@ -479,7 +467,7 @@ __device__ __forceinline__ void phase2_scalars_flat(const GP &P, const double *_
 
 template <int N, int NT, typename R, int LT, int TH>
 __device__ __forceinline__ void phase2_momentum_flat(const GP &P, const double *__restrict__ U,
-                                                     const double *__restrict__ Pr, const double *__restrict__ T1,
+                                                     const double *__restrict__ Pr, const double *__restrict__ C1,
                                                      double *__restrict__ C, const int L0, const int IF, double *sm)
 {
   using CF = P2Flat<N, NT, R, LT>;
@@ -510,7 +498,8 @@ __device__ __forceinline__ void phase2_momentum_flat(const GP &P, const double *
   if (act) {
     const int g = P.glob[IF * DoF + ID];
     const double *Ug = U + (size_t)nz * g + l;
-    const CT *T = reinterpret_cast<const CT *>(T1) + (size_t)nz * g + l;
+    R ca[4];
+    cache_sums<MIX, 0, 4>(P, C1, IF * DoF + ID, l, ca);
     rho = Ug[0]; u = Ug[fs]; v = Ug[2 * fs]; wh = Ug[3 * fs];
     const double *pg = Pr + (size_t)nz * g + l;
     pr = pg[0];
@@ -524,10 +513,10 @@ __device__ __forceinline__ void phase2_momentum_flat(const GP &P, const double *
       ua = Ug[fs + 1]; va = Ug[2 * fs + 1]; pa = pg[1];
       sa = zr + Ug[1] * P.zl[l + 1];
     }
-    rm = P.rmg[g];
+    rm = hn[H_RM * DoF];
     const double a11 = hn[H_11 * DoF], a12 = hn[H_12 * DoF], a21 = hn[H_21 * DoF], a22 = hn[H_22 * DoF];
     const R h11 = (R)a11, h12 = (R)a12, h21 = (R)a21, h22 = (R)a22;
-    const R c1 = T[0], c2 = T[fs], c3 = T[2 * fs], c4 = T[3 * fs];
+    const R c1 = ca[0], c2 = ca[1], c3 = ca[2], c4 = ca[3];
     SP(0) = h11 * c2 - h12 * c1;       // Curl12(Cache1, Cache2)
     SP(1) = h21 * c2 - h22 * c1;
     SP(2) = h11 * c3 + h12 * c4;       // Contra12(Cache3, Cache4)
@@ -675,29 +664,30 @@ __device__ __forceinline__ void phase2_momentum_flat(const GP &P, const double *
 // item: 2 * tile + role (even: momentum, odd: scalars); TH: threads of the block
 template <int N, int NT, typename R, int LT = p2_levels<N>(), int TH = P2Flat<N, NT, R, LT>::THREADS>
 __device__ __forceinline__ void phase2_flat(const GP &P, const double *__restrict__ U, const double *__restrict__ Pr,
-                                            const double *__restrict__ T1, double *__restrict__ C, const int item,
+                                            const double *__restrict__ C1, double *__restrict__ C, const int item,
                                             const int IF)
 {
   extern __shared__ double sm[];
   const int L0 = (item >> 1) * LT;
-  if (item & 1) phase2_scalars_flat<N, NT, R, LT, TH>(P, U, T1, C, L0, IF, sm);
-  else phase2_momentum_flat<N, NT, R, LT, TH>(P, U, Pr, T1, C, L0, IF, sm);
+  if (item & 1) phase2_scalars_flat<N, NT, R, LT, TH>(P, U, C1, C, L0, IF, sm);
+  else phase2_momentum_flat<N, NT, R, LT, TH>(P, U, Pr, C1, C, L0, IF, sm);
 }
 
 template <int N, int NT, typename R>
 __global__ void __launch_bounds__(HV1Tile<N, R>::THREADS, HV1Tile<N, R>::MINB)
-    k_hypervisc1_flat(const GP P, const double *__restrict__ U, double *__restrict__ C)
+    k_hypervisc1_flat(const GP P, const double *__restrict__ U, double *__restrict__ C, double *__restrict__ Pr)
 {
   extern __shared__ __align__(16) unsigned char hv1_dyn[];
-  hypervisc1_flat<N, NT, R, HV1Tile<N, R>::LT>(P, U, C, blockIdx.x, P.IF0 + blockIdx.y, reinterpret_cast<R *>(hv1_dyn));
+  hypervisc1_flat<N, NT, R, HV1Tile<N, R>::LT>(P, U, C, Pr, blockIdx.x, P.IF0 + blockIdx.y,
+                                               reinterpret_cast<R *>(hv1_dyn));
 }
 
 template <int N, int NT, typename R>
 __global__ void __launch_bounds__(P2Flat<N, NT, R>::THREADS, P2Flat<N, NT, R>::MINB)
     k_phase2_flat(const GP P, const double *__restrict__ U, const double *__restrict__ Pr,
-                  const double *__restrict__ T1, double *__restrict__ C)
+                  const double *__restrict__ C1, double *__restrict__ C)
 {
-  phase2_flat<N, NT, R>(P, U, Pr, T1, C, blockIdx.x, P.IF0 + blockIdx.y);
+  phase2_flat<N, NT, R>(P, U, Pr, C1, C, blockIdx.x, P.IF0 + blockIdx.y);
 }
 
 }  // namespace cgd

@@ -80,6 +80,9 @@ enum {
   // kR, kL of the left state and kL, kR of the right state
   C_RK0, C_RK1, C_RK2, C_RK3
 };
+// flat product grids (cgd_flat.cuh): horizontal factors of an element node:
+// dXdxI(1:2,1:2) and J over z(l), z / J, dXdxI(3,3), 2*Omega*sin(lat), z / M
+enum { H_11 = 0, H_12, H_21, H_22, H_RJ, H_J, H_33, H_FC, H_RM, H_N };
 constexpr int MAXTR = 4;
 constexpr int MAXNV = 5 + MAXTR;
 
@@ -95,6 +98,12 @@ struct GP {
   const int *inv_ptr;       // NumG + 1
   const long long *inv_off; // (IF*NC*DoF + ID)*nz for every contributor
   const long long *inv_tab; // 4 per DOF: its first four inv_off entries, -1 past the count (-1 first: > 4)
+  const int4 *etab;         // per element node the inv_tab row of its DOF, in units of nz
+  const unsigned char *own; // per element node: 1 at the DOF's first contributor of this process
+  int flat;                 // the grid is a flat product grid: the next two hold its factors
+  const double *hm;         // [IF][H_N][ID]
+  const double *zl;         // [6+2N][nz]: z (layer thickness over the first), 1/z, RecU4 coefficients (4),
+                            // slope residue of node index I (N: sum of the layer's nodes; N: half the difference over z)
   double D[25], DW[25];     // D[i + N*j] = DS[i,j]
   const double *pref;       // mixed form: per-level FP64 reference pressure and theta
   const double *thref;
@@ -197,10 +206,20 @@ struct HV1Tile {
   static constexpr int MINB = WIDE ? 3 : 4;
 };
 
+// Phase 1 also forms the pressure (Pr, unless null): rho*theta is at hand, and
+// the exp and log run beside a kernel that the shared-memory pipe bounds.  A
+// DOF's value is written by its first element node.  A kernel of its own took
+// 0.041 ms per stage on the drop-in grid (now 0.027 ms more in phase 1) and 6 of
+// 150 us per step on the smallest configurations.
+__device__ __forceinline__ void stage_pressure(const GP &P, double *Pr, int n, int g, int l, double rhoth)
+{
+  if (Pr && P.own[n]) Pr[l + (size_t)P.nz * g] = pressure_dry(P, rhoth);
+}
+
 // sbuf: the shared arrays (a kernel's dynamic buffer)
 template <int N, int NT, typename R, int LT = 256 / (N * N)>
 __device__ __forceinline__ void hypervisc1_body(const GP &P, const double *__restrict__ U, double *__restrict__ C,
-                                                const int tile, const int IF, R *sbuf)
+                                                double *__restrict__ Pr, const int tile, const int IF, R *sbuf)
 {
   constexpr bool MIX = sizeof(R) == sizeof(float);
   constexpr int DoF = N * N, RS = HV1Smem<N, NT, R, LT>::RS;
@@ -242,6 +261,7 @@ __device__ __forceinline__ void hypervisc1_body(const GP &P, const double *__res
 #pragma unroll
     for (int q = 0; q < NT; ++q) s[9 + 3 * q][si] = (R)(Ug[(5 + q) * fs] / Ug[0]);
     MCD = P.M[l + (size_t)nz * g] + P.M[l + (size_t)nz * (g + (size_t)NumG)];
+    stage_pressure(P, Pr, IF * DoF + ID, g, l, Ug[4 * fs]);
   }
   const R Js = (R)JsD, MC = (R)MCD;
   const R rJs = (R)(1.0 / JsD), rMC = (R)(1.0 / MCD);
@@ -327,10 +347,10 @@ __device__ __forceinline__ void hypervisc1_body(const GP &P, const double *__res
 // Shared arrays: HV1Smem<N, NT, R, HV1Tile<N, R>::LT>::BYTES of dynamic shared memory.
 template <int N, int NT, typename R>
 __global__ void __launch_bounds__(HV1Tile<N, R>::THREADS, HV1Tile<N, R>::MINB)
-    k_hypervisc1(const GP P, const double *__restrict__ U, double *__restrict__ C)
+    k_hypervisc1(const GP P, const double *__restrict__ U, double *__restrict__ C, double *__restrict__ Pr)
 {
   extern __shared__ __align__(16) unsigned char hv1_dyn[];
-  hypervisc1_body<N, NT, R, HV1Tile<N, R>::LT>(P, U, C, blockIdx.x, P.IF0 + blockIdx.y,
+  hypervisc1_body<N, NT, R, HV1Tile<N, R>::LT>(P, U, C, Pr, blockIdx.x, P.IF0 + blockIdx.y,
                                                reinterpret_cast<R *>(hv1_dyn));
 }
 
@@ -340,12 +360,6 @@ template <bool C32>
 __device__ __forceinline__ double cload(const double *C, long long i)
 {
   return C32 ? (double)reinterpret_cast<const float *>(C)[i] : C[i];
-}
-template <bool C32>
-__device__ __forceinline__ void cstore(double *C, long long i, double v)
-{
-  if (C32) reinterpret_cast<float *>(C)[i] = (float)v;
-  else C[i] = v;
 }
 
 // Sum over the NQ contributors (element-node offsets o) of one global DOF at
@@ -432,32 +446,54 @@ __device__ __forceinline__ void gather_node(const GP &P, const double *__restric
 // Owner gather (DSS): out(l, g, f) = sum over contributors in ascending
 // (element, node) order.  Thread per (g, l), level fastest.
 // ---------------------------------------------------------------------------
-// OUTC: the output is the phase-1 cache (stored like the contributions),
-// otherwise an FP64 tendency.
-template <bool WSPLIT, bool OUTC, bool C32>
-__device__ __forceinline__ void gather_body(const GP &P, const double *__restrict__ C, double *__restrict__ out,
-                                            const long long tid)
-{
-  const int nz = P.nz;
-  if (tid >= (long long)nz * P.NumG) return;
-  const int g = (int)(tid / nz), l = (int)(tid % nz);
-  const size_t fstr = (size_t)P.DoF * nz;
-  double acc[MAXNV];
-  gather_node<WSPLIT, C32>(P, C, g, l, fstr, acc);
-#pragma unroll
-  for (int f = 0; f < MAXNV; ++f)
-    if (f < P.NV) {
-      const long long o = l + (long long)nz * (g + (long long)P.NumG * f);
-      if (OUTC) cstore<C32>(out, o, acc[f]);
-      else out[o] = acc[f];
-    }
-}
-
-template <bool WSPLIT, bool OUTC, bool C32>
+template <bool WSPLIT, bool C32>
 __global__ void __launch_bounds__(256) k_gather(const GP P, const double *__restrict__ C,
                                                 double *__restrict__ out)
 {
-  gather_body<WSPLIT, OUTC, C32>(P, C, out, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+  const int nz = P.nz;
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (tid >= (long long)nz * P.NumG) return;
+  const int g = (int)(tid / nz), l = (int)(tid % nz);
+  double acc[MAXNV];
+  gather_node<WSPLIT, C32>(P, C, g, l, (size_t)P.DoF * nz, acc);
+#pragma unroll
+  for (int f = 0; f < MAXNV; ++f)
+    if (f < P.NV) out[l + (long long)nz * (g + (long long)P.NumG * f)] = acc[f];
+}
+
+// The DSS'd phase-1 cache of element node n (= IF*DoF + ID) at level l, fields
+// F0 .. F0+NF-1, summed from the contributions C1 as gather_node sums them
+// (ascending contributors, from 0.0; the mixed form rounds the sum to FP32).
+// Phase 2 forms it itself: 1.96 contributor reads an element node, mostly from
+// L2, instead of a kernel that wrote the summed cache (0.11 ms per stage on the
+// drop-in grid) and its read.
+template <bool C32, int F0, int NFLD, typename R>
+__device__ __forceinline__ void cache_sums(const GP &P, const double *__restrict__ C1, int n, int l, R *c)
+{
+  using CT = typename std::conditional<C32, float, double>::type;
+  const CT *C = reinterpret_cast<const CT *>(C1);
+  const size_t fstr = (size_t)P.DoF * P.nz;
+  const int4 e = P.etab[n];
+  if (e.x >= 0) {
+    const CT *p0 = C + (size_t)e.x * P.nz + l, *p1 = C + (size_t)max(e.y, 0) * P.nz + l;
+    const CT *p2 = C + (size_t)max(e.z, 0) * P.nz + l, *p3 = C + (size_t)max(e.w, 0) * P.nz + l;
+#pragma unroll
+    for (int f = 0; f < NFLD; ++f) {
+      const size_t o = (F0 + f) * fstr;
+      const double x0 = p0[o];
+      const double x1 = e.y >= 0 ? (double)p1[o] : 0.0, x2 = e.z >= 0 ? (double)p2[o] : 0.0;
+      const double x3 = e.w >= 0 ? (double)p3[o] : 0.0;
+      c[f] = (R)((((0.0 + x0) + x1) + x2) + x3);
+    }
+    return;
+  }
+  const int g = P.glob[n];
+#pragma unroll
+  for (int f = 0; f < NFLD; ++f) {
+    double a = 0.0;
+    for (int q = P.inv_ptr[g]; q < P.inv_ptr[g + 1]; ++q) a += (double)C[P.inv_off[q] + l + (F0 + f) * fstr];
+    c[f] = (R)a;
+  }
 }
 
 // ---------------------------------------------------------------------------

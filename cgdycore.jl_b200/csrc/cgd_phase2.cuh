@@ -66,6 +66,30 @@ __device__ __forceinline__ R fsum2(R acc, R c1, R x1, R c2, R x2)
 #endif
 }
 
+// RecU4's limiter max(0, min(r, min(k r + c, 1))) (OperatorKernel.jl:1044-1059)
+// with selects that keep the reference's values for every r, a NaN r giving
+// NaN, at a third of the instructions of cgd_min/cgd_max.
+__device__ __forceinline__ double upwind_limit(double r, double k, double c)
+{
+  const double lin = k * r + c;
+  const double m2 = lin > 1.0 ? 1.0 : lin;
+  const double m1 = m2 < r ? m2 : r;
+  return m1 <= 0.0 ? 0.0 : m1;
+}
+
+// The limited upwind flux of one interface, 0.25 ((|w| + w) cFL + (-|w| + w) cFR):
+// one of the two factors is zero and the other 2 w, so only the upwind side's
+// reconstruction is formed (the same value: the factors are exact).  c: the
+// ratios of the node, rows rs apart; u1, d1 the rows of the upwind and the
+// downwind level, u2 the row beyond the upwind one.
+__device__ __forceinline__ double upwind_flux(const double *c, int rs, int u1, int d1, int u2, double kc, double ks,
+                                              double w)
+{
+  const double c1 = c[u1 * rs], dc = c[d1 * rs] - c1;
+  const double r = (c1 - c[u2 * rs]) / (dc + 1.e-20);
+  return 0.5 * (w * (c1 + upwind_limit(r, ks, kc) * dc));
+}
+
 // A load the compiler may not merge with an earlier one of the same address:
 // the metric of a thread's node is read again (from L1) where it is needed
 // instead of being held in registers across a barrier.
@@ -124,7 +148,7 @@ __device__ __forceinline__ unsigned block_lanes()
 
 template <int N, int NT, typename R, int LT, int TH>
 __device__ __forceinline__ void phase2_scalars(const GP &P, const double *__restrict__ U,
-                                               const double *__restrict__ T1, double *__restrict__ C, const int L0,
+                                               const double *__restrict__ C1, double *__restrict__ C, const int L0,
                                                const int IF, double *sm)
 {
   using CF = P2Cfg<N, NT, R, LT>;
@@ -156,7 +180,8 @@ __device__ __forceinline__ void phase2_scalars(const GP &P, const double *__rest
   if (act) {
     const int g = P.glob[IF * DoF + ID];
     const double *Ug = U + (size_t)nz * g + l;
-    const CT *T = reinterpret_cast<const CT *>(T1) + (size_t)nz * g + l;
+    R ca[NS];
+    cache_sums<MIX, 4, NS>(P, C1, IF * DoF + ID, l, ca);
     rho = Ug[0];
     const double u = Ug[fs], v = Ug[2 * fs], wh = Ug[3 * fs], wm = l > 0 ? Ug[3 * fs - 1] : 0.0;
     d11s = mt[C_D11_0 * cs] + mt[C_D11_1 * cs];
@@ -167,7 +192,7 @@ __device__ __forceinline__ void phase2_scalars(const GP &P, const double *__rest
     MCD = P.M[l + (size_t)nz * g] + P.M[l + (size_t)nz * (g + (size_t)NumG)];
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
-      sc[q * PL + si] = (R)T[(4 + q) * fs];
+      sc[q * PL + si] = ca[q];
       const double c = Ug[(4 + q) * fs] / rho;
       cth[(q * CR + lvl + 2) * RS + ID] = c;
       if (MIX) sq[q * PL + si] = (R)c;
@@ -197,24 +222,16 @@ __device__ __forceinline__ void phase2_scalars(const GP &P, const double *__rest
   __syncthreads();
 
   // ---------------- vertical fluxes of interface l ----------------
-  // wCon and the limited upwind fluxes (RecU4, OperatorKernel.jl:1044-1059,
-  // J-only coefficients precomputed) between levels il and il + 1, row pl of
-  // the ratios holding level il, m the metric of that level
+  // wCon and the limited upwind fluxes between levels il and il + 1, row pl
+  // of the ratios holding level il, m the metric of that level
   auto fluxes = [&](int il, int pl, int n, const double *m, double wCon, double *f) {
-    const double kR1 = m[C_RK0 * cs], kL1 = m[C_RK1 * cs], kL2 = m[C_RK2 * cs], kR2 = m[C_RK3 * cs];
-    const int pm = il > 0 ? pl - 1 : pl, pp2 = il + 2 < nz ? pl + 2 : pl + 1;
-    const double aw = fabs(wCon);
+    const bool up = wCon > 0.0;
+    const double kc = m[(up ? C_RK0 : C_RK2) * cs], ks = m[(up ? C_RK1 : C_RK3) * cs];
+    const int far = up ? (il > 0 ? pl - 1 : pl) : (il + 2 < nz ? pl + 2 : pl + 1);
     f[0] = wCon;
 #pragma unroll
-    for (int q = 0; q < NS; ++q) {
-      const double *c = cth + (size_t)q * CR * RS + n;
-      const double cLL = c[pm * RS], cL = c[pl * RS], cR = c[(pl + 1) * RS], cRR = c[pp2 * RS];
-      double r = (cL - cLL) / (cR - cL + 1.e-20);
-      const double cFL = cL + cgd_max(0.0, cgd_min(r, cgd_min(kL1 * r + kR1, 1.0))) * (cR - cL);
-      r = (cR - cRR) / (cL - cR + 1.e-20);
-      const double cFR = cR + cgd_max(0.0, cgd_min(r, cgd_min(kR2 * r + kL2, 1.0))) * (cL - cR);
-      f[1 + q] = 0.25 * ((aw + wCon) * cFL + (-aw + wCon) * cFR);
-    }
+    for (int q = 0; q < NS; ++q)
+      f[1 + q] = upwind_flux(cth + (size_t)q * CR * RS + n, RS, up ? pl : pl + 1, up ? pl + 1 : pl, far, kc, ks, wCon);
   };
   const unsigned lanes = block_lanes<TH>();
   double Ft[1 + NS];
@@ -332,7 +349,7 @@ __device__ __forceinline__ void phase2_scalars(const GP &P, const double *__rest
 
 template <int N, int NT, typename R, int LT, int TH>
 __device__ __forceinline__ void phase2_momentum(const GP &P, const double *__restrict__ U,
-                                                const double *__restrict__ Pr, const double *__restrict__ T1,
+                                                const double *__restrict__ Pr, const double *__restrict__ C1,
                                                 double *__restrict__ C, const int L0, const int IF, double *sm)
 {
   using CF = P2Cfg<N, NT, R, LT>;
@@ -362,7 +379,8 @@ __device__ __forceinline__ void phase2_momentum(const GP &P, const double *__res
   if (act) {
     g = P.glob[IF * DoF + ID];
     const double *Ug = U + (size_t)nz * g + l;
-    const CT *T = reinterpret_cast<const CT *>(T1) + (size_t)nz * g + l;
+    R ca[4];
+    cache_sums<MIX, 0, 4>(P, C1, IF * DoF + ID, l, ca);
     rho = Ug[0]; u = Ug[fs]; v = Ug[2 * fs]; wh = Ug[3 * fs];
     pr = Pr[l + (size_t)nz * g];
     const double c110 = mt[C_D11_0 * cs], c111 = mt[C_D11_1 * cs], c120 = mt[C_D12_0 * cs], c121 = mt[C_D12_1 * cs];
@@ -373,7 +391,7 @@ __device__ __forceinline__ void phase2_momentum(const GP &P, const double *__res
     wl = l == 0 ? -(e310 * u + e320 * v) / e330 : Ug[3 * fs - 1];
     {
       const R d11 = (R)(c110 + c111), d12 = (R)(c120 + c121), d21 = (R)(c210 + c211), d22 = (R)(c220 + c221);
-      const R c1 = T[0], c2 = T[fs], c3 = T[2 * fs], c4 = T[3 * fs];
+      const R c1 = ca[0], c2 = ca[1], c3 = ca[2], c4 = ca[3];
       SP(0) = d11 * c2 - d12 * c1;       // Curl12(Cache1, Cache2)
       SP(1) = d21 * c2 - d22 * c1;
       SP(2) = d11 * c3 + d12 * c4;       // Contra12(Cache3, Cache4)
@@ -674,21 +692,21 @@ __device__ __forceinline__ void phase2_momentum(const GP &P, const double *__res
 // item: 2 * tile + role (even: momentum, odd: scalars); TH: threads of the block
 template <int N, int NT, typename R, int LT = p2_levels<N>(), int TH = P2Cfg<N, NT, R, LT>::THREADS>
 __device__ __forceinline__ void phase2_body(const GP &P, const double *__restrict__ U, const double *__restrict__ Pr,
-                                            const double *__restrict__ T1, double *__restrict__ C, const int item,
+                                            const double *__restrict__ C1, double *__restrict__ C, const int item,
                                             const int IF)
 {
   extern __shared__ double sm[];
   const int L0 = (item >> 1) * LT;
-  if (item & 1) phase2_scalars<N, NT, R, LT, TH>(P, U, T1, C, L0, IF, sm);
-  else phase2_momentum<N, NT, R, LT, TH>(P, U, Pr, T1, C, L0, IF, sm);
+  if (item & 1) phase2_scalars<N, NT, R, LT, TH>(P, U, C1, C, L0, IF, sm);
+  else phase2_momentum<N, NT, R, LT, TH>(P, U, Pr, C1, C, L0, IF, sm);
 }
 
 template <int N, int NT, typename R>
 __global__ void __launch_bounds__(P2Cfg<N, NT, R>::THREADS, P2Cfg<N, NT, R>::MINB)
-    k_phase2(const GP P, const double *__restrict__ U, const double *__restrict__ Pr, const double *__restrict__ T1,
+    k_phase2(const GP P, const double *__restrict__ U, const double *__restrict__ Pr, const double *__restrict__ C1,
              double *__restrict__ C)
 {
-  phase2_body<N, NT, R>(P, U, Pr, T1, C, blockIdx.x, P.IF0 + blockIdx.y);
+  phase2_body<N, NT, R>(P, U, Pr, C1, C, blockIdx.x, P.IF0 + blockIdx.y);
 }
 
 }  // namespace cgd

@@ -120,6 +120,15 @@ int cgd_create_part(const cgd_config *cfg, const int64_t *glob, const double *DS
                     const double *dXdxI, const double *J, const double *X, const double *M, const double *dz,
                     const cgd_halo *halo, cgd_handle **out);
 
+/* The layer-thickness ratios z(l) / z(0) (nz values, host memory) that the
+ * fast build's flat-grid kernels use.  By default a handle takes them from its
+ * first element: the sum of J's first node over the element's nodes at level l
+ * over that at level 0.  A rank of a decomposed grid is given those of the whole
+ * grid's first element, so that its contributions are the single-process ones
+ * bit for bit.  z > 0; the factors are formed and checked again.  No effect in
+ * the exact build.  No counterpart in the reference. */
+int cgd_set_layers(cgd_handle *h, const double *z);
+
 /* The exchange of one DSS point, supplied by the caller (e.g. NCCL peer
  * sends/receives between processes): nf contribution fields of nz levels per
  * element node are packed in `send` (neighbour i's items from
