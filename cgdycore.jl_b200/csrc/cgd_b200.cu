@@ -380,11 +380,10 @@ ColArgs step_args(cgd_handle *h, double *U, double dt)
   a.Vn = U;
   a.k1 = h->k1;
   a.k2 = h->k2;
-  a.dt = dt;
-  a.fac = dt * h->rk.gamma;
   a.rk = h->rk;
   a.C = h->C;
   a.jbg = h->jbg;
+  a.dt = dt;
   return a;
 }
 
@@ -405,6 +404,7 @@ void stage_piece(cgd_handle *h, double *U, const ColArgs &a0, int stage, int pie
     ColArgs a = a0;
     a.Vs = Vsrc;
     a.ps = h->pres;
+    a.set_dt(stage, a0.dt, a0.dt * h->rk.gamma);
     if (stage == 0) {
       a.kout = h->k1; a.Vout = h->Vst;
       column<0>(h, a);
@@ -1149,8 +1149,7 @@ static int schur_solve_with(cgd_handle *h, double *k, double *v, const Bands4 &b
   a.v = vd;
   a.kout = kd;
   for (int i = 0; i < 4; ++i) a.jb4[i] = b.b[i];
-  a.fac = fac;
-  a.dt = fac;
+  a.set_dt(3, fac, fac);
   column<3>(h, a);
   size_t bytes = (size_t)h->nz * h->NumG * h->NV * 8;
   if (!kdev) CK(cudaMemcpyAsync(k, kd, bytes, cudaMemcpyDeviceToHost, h->stream));
@@ -1750,8 +1749,7 @@ int cgd_jac_schur_solve_noalloc(const cgd_config *cfg, const double *U, const do
   a.v = v;
   a.kout = k;
   for (int i = 0; i < 4; ++i) a.jb4[i] = b4.b[i];
-  a.fac = fac;
-  a.dt = fac;
+  a.set_dt(3, fac, fac);
   const size_t smem = (size_t)COL_WARPS * COL_ARR * P.nz * sizeof(double);
   k_column<3, false><<<(P.NumG + COL_WARPS - 1) / COL_WARPS, 32 * COL_WARPS, smem, st>>>(P, a);
   // launch errors only: the work stays ordered on the caller's stream, which
@@ -1849,9 +1847,7 @@ int record_step(cgd_handle *h, StepTape &t, const double *u0, double dt, double 
   ColArgs a{};
   a.Vn = t.u0;
   a.k1 = t.k[0];
-  a.k2 = t.k[1];
-  a.dt = dt;
-  a.fac = dt * h->rk.gamma;
+  a.k2 = COL_KSUM ? h->k2 : t.k[1];
   a.rk = h->rk;
   a.C = h->C;
   a.jbg = t.jbg;
@@ -1861,6 +1857,12 @@ int record_step(cgd_handle *h, StepTape &t, const double *u0, double dt, double 
     gather(h, h->C1, t.T1[st], false);
     phase2(h, Vs[st], t.P[st], h->C1, h->C);
     a.kout = t.k[st];
+    if (st == 1 && COL_KSUM) {
+      a.kout = h->k2;
+      a.k2out = t.k[1];
+    }
+    a.ps = t.P[st];
+    a.set_dt(st, dt, dt * h->rk.gamma);
     if (st == 0) { a.Vout = t.V2; column<0>(h, a); }
     else if (st == 1) { a.Vout = t.V3; column<1>(h, a); }
     else { a.Vout = Uout ? Uout : h->Vst; column<2>(h, a); }

@@ -81,6 +81,19 @@ __global__ void __launch_bounds__(P2Flat<N, NT, R, LT>::THREADS, P2Flat<N, NT, R
   phase2_flat<N, NT, R, LT>(c_bgp[it.m], stage == 0 ? B.U : B.Vst, B.pres, B.C1, B.C, it.x, it.y);
 }
 
+// The constants of a member's column stage (ColArgs::set_dt on the host).
+template <int MODE>
+__device__ __forceinline__ void member_dt(ColArgs &a, double dt)
+{
+  a.rk = c_brk;
+  a.dt = dt;
+  a.fac = dt * c_brk.gamma;
+  a.ifac = 1.0 / a.fac;
+  a.ifac2 = a.ifac / a.fac;
+  a.cd[0] = a.rk.c[MODE][0] / dt;
+  a.cd[1] = a.rk.c[MODE][1] / dt;
+}
+
 template <int MODE, bool C32>
 __global__ void __launch_bounds__(32 * COL_WARPS, 4) kb_column(const WItem *__restrict__ w)
 {
@@ -93,10 +106,9 @@ __global__ void __launch_bounds__(32 * COL_WARPS, 4) kb_column(const WItem *__re
   a.k2 = B.k2;
   a.jbg = B.jbg;
   a.v = nullptr;
+  a.k2out = nullptr;
   a.jb4[0] = a.jb4[1] = a.jb4[2] = a.jb4[3] = nullptr;
-  a.dt = B.dt;
-  a.fac = B.dt * c_brk.gamma;
-  a.rk = c_brk;
+  member_dt<MODE>(a, B.dt);
   a.Vs = MODE == 0 ? B.U : B.Vst;
   a.ps = B.pres;
   if (MODE == 0) { a.kout = B.k1; a.Vout = B.Vst; }
@@ -253,20 +265,21 @@ __global__ void __launch_bounds__(256, 2) kb_stage(const FusedArgs A, const int 
     a.k2 = B.k2;
     a.jbg = B.jbg;
     a.v = nullptr;
+    a.k2out = nullptr;
     a.jb4[0] = a.jb4[1] = a.jb4[2] = a.jb4[3] = nullptr;
-    a.dt = B.dt;
-    a.fac = B.dt * c_brk.gamma;
-    a.rk = c_brk;
     a.Vs = fused_stage_state(B, stage);
     a.ps = B.pres;
     if (stage == 0) {
       a.kout = B.k1; a.Vout = B.Vst;
+      member_dt<0>(a, B.dt);
       column_body<0, C32>(c_bgp[it.m], a, it.x);
     } else if (stage == 1) {
       a.kout = B.k2; a.Vout = B.Vst2;
+      member_dt<1>(a, B.dt);
       column_body<1, C32>(c_bgp[it.m], a, it.x);
     } else {
       a.kout = nullptr; a.Vout = B.U;
+      member_dt<2>(a, B.dt);
       column_body<2, C32>(c_bgp[it.m], a, it.x);
     }
     __syncthreads();

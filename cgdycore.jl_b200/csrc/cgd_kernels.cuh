@@ -515,8 +515,10 @@ __device__ __forceinline__ void cache_sums(const GP &P, const double *__restrict
 struct ColArgs {
   const double *C;       // contributions of phase 2 (MODE 0..2)
   const double *Vn;      // step initial state (MODE 0..2)
+  // MODE 1 reads k1; MODE 2 k1 and k2, or (COL_KSUM) their sum alone from k2
   const double *k1, *k2;
-  double *kout;          // MODE 0,1,3
+  double *kout;          // MODE 0,1,3 (MODE 1 with COL_KSUM: k1 + k2)
+  double *k2out;         // MODE 1 with COL_KSUM: k2 itself, for the adjoint's tape (else null)
   double *Vout;          // MODE 0,1 (stage state), 2 (new state)
   double *v;             // MODE 3: right-hand side (overwritten)
   // MODE 3: the four Jacobian bands JRhoW, JWRho, JWRhoTh, JRhoThW, each
@@ -527,8 +529,29 @@ struct ColArgs {
   // pressure (Vs may be Vout: each lane reads its own levels before writing them)
   const double *Vs, *ps;
   double dt, fac;
+  double cd[2];          // c[MODE][j] / dt
+  double ifac, ifac2;    // 1 / fac, 1 / fac / fac
   RK rk;
+
+  void set_dt(int mode, double dt_, double fac_)
+  {
+    dt = dt_;
+    fac = fac_;
+    ifac = 1.0 / fac;
+    ifac2 = ifac / fac;
+    for (int j = 0; j < 2; ++j) cd[j] = mode <= 2 ? rk.c[mode][j] / dt : 0.0;
+  }
 };
+
+// The third stage needs k1 and k2 only in c31/dt k1 + c32/dt k2, m1 k1 + m2 k2,
+// and the SSP-Knoth scheme has c31 = c32, m1 = m2 and a31 = a32
+// (src/Integration/RosenbrockMethod.jl:26-47).  The fast build's second stage
+// therefore keeps k1 + k2 instead of k2: one array less to read in the third.
+#ifdef CGD_FAST
+constexpr bool COL_KSUM = true;
+#else
+constexpr bool COL_KSUM = false;
+#endif
 
 constexpr int COL_WARPS = 8;
 // per warp: fv of rho, w, rho*theta, 8 bands, tri[3], x; each nz long.  (The
@@ -566,6 +589,28 @@ __device__ __forceinline__ void jac_bands(const GP &P, double RhoL, double RhoR,
   jb[6] = -RhoThF / dzL;           // JRhoThW[1]
   jb[7] = RhoThF / dzR;            // JRhoThW[2]
 }
+
+#ifdef CGD_FAST
+// jac_bands with reciprocals shared by its quotients: riL, riR the
+// reciprocals of dzL and dzR (two divisions instead of fifteen)
+__device__ __forceinline__ void jac_bands_rcp(const GP &P, double RhoL, double RhoR, double RhoThL, double RhoThR,
+                                              double dPdThL, double dPdThR, double dzL, double dzR, double riL,
+                                              double riR, double *jb)
+{
+  const double dzs = dzL + dzR, rs = 1.0 / dzs, num = RhoL * dzL + RhoR * dzR;
+  const double RhoF = num * rs, rF = dzs * (1.0 / num);   // rF = 1 / RhoF
+  jb[0] = -RhoF * riL;
+  jb[1] = RhoF * riR;
+  const double q = rF * rs, w = 2.0 * q, b = P.Grav * q;
+  jb[4] = -dPdThR * w;
+  jb[5] = dPdThL * w;
+  jb[2] = -b * dzR;
+  jb[3] = -b * dzL;
+  const double RhoThF = (RhoThL * dzL + RhoThR * dzR) * rs;
+  jb[6] = -RhoThF * riL;
+  jb[7] = RhoThF * riR;
+}
+#endif
 
 __device__ __forceinline__ void jac_at(const GP &P, double RhoL, double RhoR, double RhoThL0, double RhoThR0,
                                        double dzL, double dzR, double *jb)
@@ -675,6 +720,27 @@ __device__ __forceinline__ void warp_tri_solve(const double *t0, const double *t
   if (i1 < n) x[i1] = x1v;
 }
 
+// The update of the second and third stage at state entry o: k of the stage,
+// x1 = k1 (third stage with COL_KSUM: k1 + k2), x2 = k2.
+template <int MODE>
+__device__ __forceinline__ void stage_update(const ColArgs &A, size_t o, double vn, double x1, double x2, double k)
+{
+  if (MODE == 1) {
+    if (COL_KSUM) {
+      const double ks = x1 + k;
+      A.kout[o] = ks;
+      if (A.k2out) A.k2out[o] = k;
+      A.Vout[o] = vn + A.rk.a[2][0] * ks;
+    } else {
+      A.kout[o] = k;
+      A.Vout[o] = vn + A.rk.a[2][0] * x1 + A.rk.a[2][1] * k;
+    }
+  } else {
+    if (COL_KSUM) A.Vout[o] = vn + A.rk.m[0] * x1 + A.rk.m[2] * k;
+    else A.Vout[o] = vn + A.rk.m[0] * x1 + A.rk.m[1] * x2 + A.rk.m[2] * k;
+  }
+}
+
 template <int MODE, bool C32>
 __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const int bx)
 {
@@ -730,13 +796,18 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
         const size_t o = o0 + f * fs;
         double x = gacc[f];
         double x1 = 0.0, x2 = 0.0;
-        if (MODE >= 1) {
-          x1 = A.k1[o];
-          x = x + A.rk.c[MODE][0] / A.dt * x1;
-        }
-        if (MODE >= 2) {
-          x2 = A.k2[o];
-          x = x + A.rk.c[MODE][1] / A.dt * x2;
+        if (MODE == 2 && COL_KSUM) {
+          x1 = A.k2[o];
+          x = x + A.cd[0] * x1;
+        } else {
+          if (MODE >= 1) {
+            x1 = A.k1[o];
+            x = x + A.cd[0] * x1;
+          }
+          if (MODE >= 2) {
+            x2 = A.k2[o];
+            x = x + A.cd[1] * x2;
+          }
         }
         if (f == 0 || f == 3 || f == 4) {
           const int sf = f == 0 ? 0 : f - 2;   // 0, 1, 2
@@ -749,17 +820,20 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
           if (MODE == 0) {
             A.kout[o] = k;
             A.Vout[o] = vn + A.rk.a[1][0] * k;
-          } else if (MODE == 1) {
-            A.kout[o] = k;
-            A.Vout[o] = vn + A.rk.a[2][0] * x1 + A.rk.a[2][1] * k;
           } else {
-            A.Vout[o] = vn + A.rk.m[0] * x1 + A.rk.m[1] * x2 + A.rk.m[2] * k;
+            stage_update<MODE>(A, o, vn, x1, x2, k);
           }
         }
       }
       if (MODE == 0) {
         // dPresdRhoTh once per level, shared with the interface below
+#ifdef CGD_FAST
+        // Rd (Rd rhotheta / p0)^(kappa/(1-kappa)) = p / rhotheta with the pressure at hand
+        xs[l] = A.ps[o0] / A.Vn[o0 + 4 * fs];
+        tri[l] = 1.0 / P.dz[o0];
+#else
         xs[l] = dpdrhoth(P, A.Vn[o0 + 4 * fs]);
+#endif
       }
     } else {
       fv[l] = A.v[o0];
@@ -785,8 +859,13 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
       if (MODE == 0) {
         double b[8];
         const double *V0 = A.Vn + (size_t)nz * g;
+#ifdef CGD_FAST
+        jac_bands_rcp(P, V0[l], V0[l + 1], V0[l + 4 * fs], V0[l + 1 + 4 * fs], xs[l], xs[l + 1],
+                      P.dz[l + (size_t)nz * g], P.dz[l + 1 + (size_t)nz * g], tri[l], tri[l + 1], b);
+#else
         jac_bands(P, V0[l], V0[l + 1], V0[l + 4 * fs], V0[l + 1 + 4 * fs], xs[l], xs[l + 1],
                   P.dz[l + (size_t)nz * g], P.dz[l + 1 + (size_t)nz * g], b);
+#endif
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
           jb[r * LS + l] = b[r];
@@ -801,8 +880,7 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
 #define FV0(i) fv[(i)]
 #define FV3(i) fv[LS + (i)]
 #define FV4(i) fv[2 * LS + (i)]
-  const double invfac = 1.0 / fac;
-  const double invfac2 = invfac / fac;
+  const double invfac2 = A.ifac2;
   double v3new[2] = {0.0, 0.0};
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
@@ -817,7 +895,12 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
       else t2 = -JB(1, 1, l + 1) * JB(0, 1, l) - JB(2, 1, l + 1) * JB(3, 1, l);
       tri[l] = t0; tri[LS + l] = t1; tri[2 * LS + l] = t2;
       // SchurSolveFKernel!
-      v3new[it] = FV3(l) / fac + JB(1, 1, l) * FV0(l) + JB(1, 0, l) * FV0(l + 1) +
+#ifdef CGD_FAST
+      const double v3 = FV3(l) * A.ifac;
+#else
+      const double v3 = FV3(l) / fac;
+#endif
+      v3new[it] = v3 + JB(1, 1, l) * FV0(l) + JB(1, 0, l) * FV0(l + 1) +
                   JB(2, 1, l) * FV4(l) + JB(2, 0, l) * FV4(l + 1);
     }
   }
@@ -889,15 +972,10 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
         const double vn = A.Vn[o];
         A.kout[o] = k;
         A.Vout[o] = vn + A.rk.a[1][0] * k;
-      } else if (MODE == 1) {
-        const double vn = A.Vn[o];
-        A.kout[o] = k;
-        A.Vout[o] = vn + A.rk.a[2][0] * s1[it][sf] + A.rk.a[2][1] * k;
-      } else if (MODE == 2) {
+      } else if (MODE <= 2) {
         // Vout may alias Vn: this lane alone reads index o and then writes it
-        const double vn = A.Vn[o];
-        A.Vout[o] = vn + A.rk.m[0] * s1[it][sf] + A.rk.m[1] * s2[it][sf] + A.rk.m[2] * k;
-        if (A.kout) A.kout[o] = k;   // the last stage's k of rho, w, rho*theta (adjoint replay only)
+        stage_update<MODE>(A, o, A.Vn[o], s1[it][sf], s2[it][sf], k);
+        if (MODE == 2 && A.kout) A.kout[o] = k;   // the last stage's k of rho, w, rho*theta (adjoint replay only)
       } else {
         A.kout[o] = k;
       }
