@@ -265,11 +265,13 @@ class Dycore:
         chaining step adjoints backwards over checkpoints: the forward run
         keeps the state every `every` steps (default: checkpoint_every), and
         the reverse sweep takes the segments from the last to the first.
-        With tape (default: when a segment's recorded steps fit in
-        mem_budget), each segment is re-run from its checkpoint recording
-        every step (tape_record_step) and the step adjoints read the
-        records; otherwise the segment's states are kept and each step
-        adjoint replays its step (ros_step_adjoint).  At most nsteps/every
+        With tape (default: when segments have more than one step and a
+        segment's recorded steps fit in mem_budget), each segment is re-run
+        from its checkpoint recording every step (tape_record_step) and the
+        step adjoints read the records; otherwise the segment's states are
+        kept and each step adjoint replays its step (ros_step_adjoint).  A
+        segment of one step is re-run once either way, and the replay uses the
+        handle's own records instead of allocating a tape slot.  At most nsteps/every
         checkpoints plus one segment are held.  The arrays may be host
         (numpy) or device (torch) arrays; checkpoints stay where U0 is.
         Lout may be a function of the final state U_n that returns the
@@ -277,7 +279,7 @@ class Dycore:
         nsteps = int(nsteps)
         every = self.checkpoint_every(nsteps, mem_budget) if every is None else max(1, int(every))
         if tape is None:
-            tape = every * self.tape_bytes_per_step() <= mem_budget
+            tape = every > 1 and every * self.tape_bytes_per_step() <= mem_budget
         # one working state for every forward step, so the library's captured
         # step (bound to the state's address) is reused
         checkpoints = {0: _copy(U0)}
