@@ -31,7 +31,8 @@ SRC = os.path.join(PKG_DIR, "csrc", "cgd_b200.cu")
 SRC_ADJ = os.path.join(PKG_DIR, "csrc", "cgd_adjoint.cu")
 OBJ_DIR = os.path.join(PKG_DIR, "_build")
 DEPS = [os.path.join(PKG_DIR, "csrc", f) for f in ("cgd_b200.cu", "cgd_adjoint.cu", "cgd_kernels.cuh", "cgd_phase2.cuh",
-                                                   "cgd_flat.cuh", "cgd_batch.cuh", "cgd_adjoint.cuh", "cgd_init.cuh", "cgd_output.cuh", "cgd_adjoint_launch.h")] + [
+                                                   "cgd_flat.cuh", "cgd_batch.cuh", "cgd_adjoint.cuh", "cgd_adjoint_flat.cuh",
+                                                   "cgd_init.cuh", "cgd_output.cuh", "cgd_adjoint_launch.h")] + [
     os.path.join(os.path.dirname(PKG_DIR), "include", f) for f in ("cgd_b200.h", "cgd_math.h")]
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",

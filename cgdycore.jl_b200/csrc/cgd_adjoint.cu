@@ -8,6 +8,7 @@
 // without contraction.
 #define CGD_ADJOINT_TU
 #include "cgd_adjoint.cuh"
+#include "cgd_adjoint_flat.cuh"
 #include "cgd_adjoint_launch.h"
 
 namespace cgd {
@@ -18,11 +19,20 @@ template <int N>
 cudaError_t rhs_adjoint_t(const GP &gp, const double *U, const double *T1, const double *pres, const double *LF,
                           double *LU, double *LT1, cudaStream_t stream)
 {
-  using CF = AdjCfg<N>;
-  cudaError_t e = cudaFuncSetAttribute(k_phase2_adj<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::SMEM);
-  if (e != cudaSuccess) return e;
-  const dim3 grid((gp.nz + CF::LC - 1) / CF::LC, gp.NF);
-  k_phase2_adj<N><<<grid, CF::THREADS, CF::SMEM, stream>>>(gp, U, pres, T1, LF, LU, LT1);
+  cudaError_t e;
+  if (gp.flat) {
+    using FF = AdjFlat<N>;
+    e = cudaFuncSetAttribute(k_phase2_adj_flat<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FF::SMEM);
+    if (e != cudaSuccess) return e;
+    const dim3 fgrid(2 * ((gp.nz + FF::LT - 1) / FF::LT), gp.NF);
+    k_phase2_adj_flat<N><<<fgrid, FF::THREADS, FF::SMEM, stream>>>(gp, U, pres, T1, LF, LU, LT1);
+  } else {
+    using CF = AdjCfg<N>;
+    e = cudaFuncSetAttribute(k_phase2_adj<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::SMEM);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((gp.nz + CF::LC - 1) / CF::LC, gp.NF);
+    k_phase2_adj<N><<<grid, CF::THREADS, CF::SMEM, stream>>>(gp, U, pres, T1, LF, LU, LT1);
+  }
   using HT = AdjHV1Tile<N>;
   const dim3 grid1((gp.nz + HT::LT - 1) / HT::LT, gp.NF);
   k_hypervisc1_adj<N><<<grid1, HT::THREADS, 0, stream>>>(gp, U, LT1, LU);

@@ -12,7 +12,9 @@
 // adjoints to LU once, with the level's other element nodes (global atomics,
 // runs of consecutive levels).  The general kernel (k_phase2_adj) sums them by
 // FP64 atomics in shared memory, about 50 a node and level, which are
-// compare-and-swap loops.  The levels' slope residue (1e-16 of dXdxI(3,3)) is
+// compare-and-swap loops.  nPanel 30, p 4, nz 45, no tracer: 2.33 -> 1.05 ms,
+// and the adjoint of a step 14.7 -> 9.5 ms; registers capped for two CTAs an
+// SM, with spills, beat one CTA an SM without them (10.5 ms a step).  The levels' slope residue (1e-16 of dXdxI(3,3)) is
 // not differentiated.
 #pragma once
 #include "cgd_phase2.cuh"
@@ -69,6 +71,16 @@ __device__ __forceinline__ void phase2_scalars_adj(const GP &P, const double *__
   const int g = P.glob[IF * DoF + ID];
   const double *Ug = U + (size_t)nz * g + l, *Lg = LF + (size_t)nz * g + l;
   double *Og = LU + (size_t)nz * g + l;
+  // halo: thread t < 4 DoF takes node t / 4 of level L0-2, L0-1, L0+LT or L0+LT+1
+  static_assert(4 * DoF <= TH, "one halo slot per thread");
+  const int hID = t >> 2, hr = (t & 3) < 2 ? (t & 3) : LT + (t & 3), hl = L0 - 2 + hr;
+  const bool hs = t < 4 * DoF && hl >= 0 && hl < nz;
+  double hrho = 1.0, hrth = 0.0;
+  if (hs) {
+    const double *Un = U + (size_t)nz * P.glob[IF * DoF + hID] + hl;
+    hrho = Un[0];
+    hrth = Un[4 * fs];
+  }
   double rho = 1.0, u = 0.0, v = 0.0, wh = 0.0, thl = 0.0, ar = 0.0, at = 0.0;
   if (act) {
     const double rm = hn[H_RM * DoF];
@@ -81,12 +93,7 @@ __device__ __forceinline__ void phase2_scalars_adj(const GP &P, const double *__
     s[PL + si] = at;
     s[2 * PL + si] = T1[(size_t)nz * g + l + 4 * fs];
   }
-  for (int x = t; x < 4 * DoF; x += TH) {
-    const int n = x >> 2, h = x & 3, r = h < 2 ? h : LT + h, lev = L0 - 2 + r;
-    if (lev < 0 || lev >= nz) continue;
-    const double *Un = U + (size_t)nz * P.glob[IF * DoF + n] + lev;
-    th[r * RS + n] = Un[4 * fs] / Un[0];
-  }
+  if (hs) th[hr * RS + hID] = hrth / hrho;
   // neighbours above: state and lambda over z of level l + 1
   double ra = __shfl_down_sync(lanes, rho, 1, LT), ua = __shfl_down_sync(lanes, u, 1, LT);
   double va = __shfl_down_sync(lanes, v, 1, LT), ara = __shfl_down_sync(lanes, ar, 1, LT);
