@@ -326,6 +326,19 @@ __device__ __forceinline__ void phase2_scalars_flat(const GP &P, const double *_
   const unsigned lanes = block_lanes<TH>();
 
   // ---------------- operands of the first round, vertical halo ----------------
+  // halo: thread t < 4 DoF takes node t / 4 of level L0-2, L0-1, L0+LT or
+  // L0+LT+1; its loads are issued first, beside the thread's own
+  static_assert(4 * DoF <= TH, "one halo slot per thread");
+  const int hID = t >> 2, hr = (t & 3) < 2 ? (t & 3) : LT + (t & 3), hl = L0 - 2 + hr;
+  const bool hs = t < 4 * DoF && hl >= 0 && hl < nz;
+  double hrho = 1.0, hq[NS], hw = 0.0, ha = 0.0;
+  if (hs) {
+    const double *Ug = U + (size_t)nz * P.glob[IF * DoF + hID] + hl;
+    hrho = Ug[0];
+#pragma unroll
+    for (int q = 0; q < NS; ++q) hq[q] = Ug[(4 + q) * fs];
+    if ((t & 3) == 1) { hw = Ug[3 * fs]; ha = Ug[1]; }
+  }
   double rho = 1.0, F0 = 0.0, rm = 0.0;
   R h11 = 0, h12 = 0, h21 = 0, h22 = 0;
   if (act) {
@@ -350,15 +363,11 @@ __device__ __forceinline__ void phase2_scalars_flat(const GP &P, const double *_
     scon[PL + si] = (R)(-rho * (a21 * u + a22 * v));
     h11 = (R)a11; h12 = (R)a12; h21 = (R)a21; h22 = (R)a22;
   }
-  for (int s = t; s < 4 * DoF; s += TH) {   // levels L0-2, L0-1, L0+LT, L0+LT+1
-    const int n = s >> 2, h = s & 3, r = h < 2 ? h : LT + h;
-    const int lev = L0 - 2 + r;
-    if (lev < 0 || lev >= nz) continue;
-    const double *Ug = U + (size_t)nz * P.glob[IF * DoF + n] + lev;
-    const double rh = Ug[0], rr = 1.0 / rh;
+  if (hs) {
+    const double rr = 1.0 / hrho;
 #pragma unroll
-    for (int q = 0; q < NS; ++q) cth[(q * CR + r) * RS + n] = ratio_of(Ug[(4 + q) * fs], rh, rr);
-    if (h == 1) f0[n] = Ug[3 * fs] * (rh + Ug[1]);
+    for (int q = 0; q < NS; ++q) cth[(q * CR + hr) * RS + hID] = ratio_of(hq[q], hrho, rr);
+    if ((t & 3) == 1) f0[hID] = hw * (hrho + ha);
   }
   __syncthreads();
 
@@ -678,7 +687,7 @@ __global__ void __launch_bounds__(HV1Tile<N, R>::THREADS, HV1Tile<N, R>::MINB)
     k_hypervisc1_flat(const GP P, const double *__restrict__ U, double *__restrict__ C, double *__restrict__ Pr)
 {
   extern __shared__ __align__(16) unsigned char hv1_dyn[];
-  hypervisc1_flat<N, NT, R, HV1Tile<N, R>::LT>(P, U, C, Pr, blockIdx.x, P.IF0 + blockIdx.y,
+  hypervisc1_flat<N, NT, R, HV1Tile<N, R>::LT>(P, U, C, Pr, blockIdx.x, launch_element(P),
                                                reinterpret_cast<R *>(hv1_dyn));
 }
 
@@ -687,7 +696,7 @@ __global__ void __launch_bounds__(P2Flat<N, NT, R>::THREADS, P2Flat<N, NT, R>::M
     k_phase2_flat(const GP P, const double *__restrict__ U, const double *__restrict__ Pr,
                   const double *__restrict__ C1, double *__restrict__ C)
 {
-  phase2_flat<N, NT, R>(P, U, Pr, C1, C, blockIdx.x, P.IF0 + blockIdx.y);
+  phase2_flat<N, NT, R>(P, U, Pr, C1, C, blockIdx.x, launch_element(P));
 }
 
 }  // namespace cgd

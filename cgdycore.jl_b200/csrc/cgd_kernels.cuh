@@ -90,6 +90,7 @@ constexpr int MAXNV = 5 + MAXTR;
 struct GP {
   int N, DoF, nz, NF, NumG, NumTr, NV;
   int NC;                   // contribution slots per element node: NV fields + the lower-node w of phase 2
+  int rev;                  // walk the elements or columns of a launch from the last to the first (stage_piece)
   int IF0;                  // first element of a launch over a range of elements (k_hypervisc1, k_phase2)
   const double *met;        // [IF][comp][ID][nz]
   const double *M;          // (nz, NumG, 2)
@@ -115,6 +116,12 @@ struct GP {
   const double *coslat, *sinlat;   // (NumG) latitude of each column's surface node
   const double *dampc;             // (nz, NumG) damping rate at the layer midpoint
 };
+
+// The element of a launch with one blockIdx.y per element
+__device__ __forceinline__ int launch_element(const GP &P)
+{
+  return P.IF0 + (int)(P.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y);
+}
 
 // Rosenbrock-W coefficients (src/Integration/RosenbrockMethod.jl:26-47).
 struct RK {
@@ -350,7 +357,7 @@ __global__ void __launch_bounds__(HV1Tile<N, R>::THREADS, HV1Tile<N, R>::MINB)
     k_hypervisc1(const GP P, const double *__restrict__ U, double *__restrict__ C, double *__restrict__ Pr)
 {
   extern __shared__ __align__(16) unsigned char hv1_dyn[];
-  hypervisc1_body<N, NT, R, HV1Tile<N, R>::LT>(P, U, C, Pr, blockIdx.x, P.IF0 + blockIdx.y,
+  hypervisc1_body<N, NT, R, HV1Tile<N, R>::LT>(P, U, C, Pr, blockIdx.x, launch_element(P),
                                                reinterpret_cast<R *>(hv1_dyn));
 }
 
@@ -990,7 +997,7 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
 template <int MODE, bool C32>
 __global__ void __launch_bounds__(32 * COL_WARPS, col_min_blocks<MODE>()) k_column(const GP P, const ColArgs A)
 {
-  column_body<MODE, C32>(P, A, blockIdx.x);
+  column_body<MODE, C32>(P, A, P.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
 }
 
 // The kernels below are defined by the forward translation unit only (the
