@@ -182,6 +182,23 @@ bool is_device_ptr(const void *p)
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// whether a device pointer lies in the current device's own memory
+bool on_this_device(const void *p)
+{
+  cudaPointerAttributes a;
+  int dev = -1;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == dev;
+}
+
+bool overlaps(const void *p, size_t np, const void *q, size_t nq)
+{
+  const uintptr_t a = (uintptr_t)p, b = (uintptr_t)q;
+  return a < b + nq && b < a + np;
+}
 
 // The element range of a phase-1 or phase-2 launch: all elements, or the
 // range the decomposed step set (cgd_handle::el0, neln).
@@ -1096,10 +1113,10 @@ static Bands4 handle_bands(cgd_handle *h)
   return Bands4{{h->bands, h->bands + bs, h->bands + 2 * bs, h->bands + 3 * bs}};
 }
 
-static void launch_jac(cgd_handle *h, const double *Ud, const Bands4 &out)
+static void launch_jac(cgd_handle *h, const double *Ud, const Bands4 &out, const Bands4 &out2)
 {
-  const long long n = (long long)(h->nz - 1) * h->NumG;
-  k_jac<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->gp, Ud, out);
+  const long long n = (long long)h->nz * h->NumG;
+  k_jac<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(h->gp, Ud, out, out2);
 }
 
 int cgd_jac(cgd_handle *h, const double *U, double *bands)
@@ -1109,7 +1126,7 @@ int cgd_jac(cgd_handle *h, const double *U, double *bands)
   double *Ud;
   int rc = stage_in(h, U, h->Ubuf, true, &Ud);
   if (rc) return rc;
-  launch_jac(h, Ud, handle_bands(h));
+  launch_jac(h, Ud, handle_bands(h), Bands4{});
   if (bands) {
     size_t bytes = (size_t)8 * (h->nz - 1) * h->NumG * 8;
     CK(cudaMemcpyAsync(bands, h->bands, bytes, is_device_ptr(bands) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
@@ -1130,13 +1147,24 @@ int cgd_jac_bands(cgd_handle *h, const double *U, double *JRhoW, double *JWRho, 
   double *user[4] = {JRhoW, JWRho, JWRhoTh, JRhoThW};
   bool dev[4];
   for (int i = 0; i < 4; ++i) dev[i] = is_device_ptr(user[i]);
-  // the handle's own bands (for cgd_schur_solve) and the caller's arrays
+  // the handle's own bands (for cgd_schur_solve) and the caller's arrays: the
+  // kernel writes those that lie apart in this device's memory, the others
+  // (host, another device, overlapping the state or one another) are copied
   const Bands4 hb = handle_bands(h);
-  launch_jac(h, Ud, hb);
   const size_t bytes = (size_t)2 * (h->nz - 1) * h->NumG * 8;
+  Bands4 direct{};
+  for (int i = 0; i < 4; ++i) {
+    bool apart = dev[i] && on_this_device(user[i]) && (uintptr_t)user[i] % sizeof(double) == 0 &&
+                 !overlaps(user[i], bytes, Ud, (size_t)h->nz * h->NumG * h->NV * 8) &&
+                 !overlaps(user[i], bytes, h->bands, 4 * bytes);
+    for (int j = 0; j < 4; ++j) apart = apart && (j == i || !overlaps(user[i], bytes, user[j], bytes));
+    if (apart) direct.b[i] = user[i];
+  }
+  launch_jac(h, Ud, hb, direct);
   for (int i = 0; i < 4; ++i)
-    CK(cudaMemcpyAsync(user[i], hb.b[i], bytes, dev[i] ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                       h->stream));
+    if (!direct.b[i])
+      CK(cudaMemcpyAsync(user[i], hb.b[i], bytes, dev[i] ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                         h->stream));
   rc = finish(h);
   if (!rc) h->have_bands = true;
   return rc;
@@ -1746,10 +1774,10 @@ int cgd_jac_schur_solve_noalloc(const cgd_config *cfg, const double *U, const do
   GP P{};
   P.nz = cfg->nz; P.NumG = cfg->NumG; P.NumTr = cfg->NumTr; P.NV = 5 + cfg->NumTr; P.NC = P.NV + 1;
   P.dz = dz; P.Grav = cfg->Grav; P.Rd = cfg->Rd; P.p0 = cfg->p0; P.kappa = cfg->Rd / cfg->Cpd;
-  const long long n = (long long)(P.nz - 1) * P.NumG;
+  const long long n = (long long)P.nz * P.NumG;
   const size_t bs = (size_t)2 * (P.nz - 1) * P.NumG;
   const Bands4 b4{{bands, bands + bs, bands + 2 * bs, bands + 3 * bs}};
-  k_jac<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(P, U, b4);
+  k_jac<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(P, U, b4, Bands4{});
   ColArgs a{};
   a.v = v;
   a.kout = k;

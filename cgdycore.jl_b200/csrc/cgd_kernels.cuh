@@ -619,12 +619,6 @@ __device__ __forceinline__ void jac_bands_rcp(const GP &P, double RhoL, double R
 }
 #endif
 
-__device__ __forceinline__ void jac_at(const GP &P, double RhoL, double RhoR, double RhoThL0, double RhoThR0,
-                                       double dzL, double dzR, double *jb)
-{
-  jac_bands(P, RhoL, RhoR, RhoThL0, RhoThR0, dpdrhoth(P, RhoThL0), dpdrhoth(P, RhoThR0), dzL, dzR, jb);
-}
-
 // Solve M x = b for one column with the warp's 32 lanes (the fast build's
 // triSolve!).  M(i,i) = t1(i), M(i+1,i) = t2(i), M(i,i+1) = t0(i+1), n <= 64
 // rows; lane L holds rows 2L and 2L+1.  The Thomas recurrences become scans:
@@ -1057,21 +1051,35 @@ __global__ void __launch_bounds__(256) k_physics(const GP P, const double *__res
   F[t + 4 * S] = f[4];
 }
 
-// Jacobian bands into memory (cgd_jac): one thread per (interface, column)
-__global__ void k_jac(const GP P, const double *__restrict__ U, const Bands4 out)
+// Jacobian bands into memory (cgd_jac): one thread per (level, column), which
+// evaluates dp/d(rho theta) of its level and takes the upper level's from the
+// next thread, and writes the bands of the interface above; out2 (null
+// entries: none) takes a copy for the caller.  nPanel 20, nz 37: 47 us and four
+// copies of the bands before.
+__global__ void __launch_bounds__(256) k_jac(const GP P, const double *__restrict__ U, const Bands4 out,
+                                             const Bands4 out2)
 {
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = P.nz - 1;
-  if (tid >= (long long)n * P.NumG) return;
-  const int g = (int)(tid / n), l = (int)(tid % n);
-  const int nz = P.nz;
-  const size_t fs = (size_t)nz * P.NumG;
-  const double *V0 = U + (size_t)nz * g;
+  __shared__ double dp[257];
+  const int nz = P.nz, n = nz - 1, t = threadIdx.x;
+  const long long tid = (long long)blockIdx.x * 256 + t, S = (long long)nz * P.NumG;
+  const bool in = tid < S;
+  if (in) dp[t] = dpdrhoth(P, U[tid + 4 * S]);
+  if (t == 255 && tid + 1 < S) dp[256] = dpdrhoth(P, U[tid + 1 + 4 * S]);
+  __syncthreads();
+  if (!in) return;
+  const long long g = tid / nz;
+  const int l = (int)(tid - g * nz);
+  if (l == n) return;
   double b[8];
-  jac_at(P, V0[l], V0[l + 1], V0[l + 4 * fs], V0[l + 1 + 4 * fs], P.dz[l + (size_t)nz * g],
-         P.dz[l + 1 + (size_t)nz * g], b);
+  jac_bands(P, U[tid], U[tid + 1], U[tid + 4 * S], U[tid + 1 + 4 * S], dp[t], dp[t + 1], P.dz[tid], P.dz[tid + 1], b);
+  const size_t o = 2 * (l + (size_t)n * g);
+#pragma unroll
   for (int arr = 0; arr < 4; ++arr)
-    for (int r = 0; r < 2; ++r) out.b[arr][r + 2 * (l + (size_t)n * g)] = b[arr * 2 + r];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      out.b[arr][o + r] = b[arr * 2 + r];
+      if (out2.b[arr]) out2.b[arr][o + r] = b[arr * 2 + r];
+    }
 }
 
 __device__ __forceinline__ void pressure_body(const GP &P, const double *__restrict__ U, double *__restrict__ p,
