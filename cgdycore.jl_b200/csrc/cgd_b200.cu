@@ -345,11 +345,11 @@ void gather(cgd_handle *h, const double *C, double *out, bool wsplit)
 template <int MODE, bool C32>
 void column_t(cgd_handle *h, const ColArgs &a)
 {
-  size_t smem = (size_t)COL_WARPS * COL_ARR * h->nz * sizeof(double);
+  size_t smem = (size_t)COL_WARPS * COL_ARR<MODE> * h->nz * sizeof(double);
   static std::atomic<unsigned long long> attr{0};
-  if (first_on_device(attr)) {   // up to 8 warps x 15 arrays x 64 levels
+  if (first_on_device(attr)) {
     cudaFuncSetAttribute(k_column<MODE, C32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         COL_WARPS * COL_ARR * 64 * (int)sizeof(double));
+                         COL_WARPS * COL_ARR_MAX * 64 * (int)sizeof(double));
   }
   k_column<MODE, C32><<<(h->NumG + COL_WARPS - 1) / COL_WARPS, 32 * COL_WARPS, smem, h->stream>>>(h->gp, a);
 }
@@ -1765,7 +1765,7 @@ int cgd_jac_schur_solve_noalloc(const cgd_config *cfg, const double *U, const do
       void *p = nullptr;
       CK(cudaGetSymbolAddress(&p, g_noalloc_scratch));
       CK(cudaFuncSetAttribute(k_column<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              COL_WARPS * COL_ARR * 64 * (int)sizeof(double)));
+                              COL_WARPS * COL_ARR_MAX * 64 * (int)sizeof(double)));
       g_noalloc_ptr[dev] = static_cast<double *>(p);
     }
     bands = g_noalloc_ptr[dev];
@@ -1783,7 +1783,7 @@ int cgd_jac_schur_solve_noalloc(const cgd_config *cfg, const double *U, const do
   a.kout = k;
   for (int i = 0; i < 4; ++i) a.jb4[i] = b4.b[i];
   a.set_dt(3, fac, fac);
-  const size_t smem = (size_t)COL_WARPS * COL_ARR * P.nz * sizeof(double);
+  const size_t smem = (size_t)COL_WARPS * COL_ARR<3> * P.nz * sizeof(double);
   k_column<3, false><<<(P.NumG + COL_WARPS - 1) / COL_WARPS, 32 * COL_WARPS, smem, st>>>(P, a);
   // launch errors only: the work stays ordered on the caller's stream, which
   // the caller synchronises (or orders further work on) itself
@@ -2262,7 +2262,7 @@ void batch_enqueue_t(cgd_batch *b, WItem *const *w, bool p2alt)
   constexpr bool C32 = sizeof(R) == sizeof(float);
   constexpr size_t hsmem = HV1Smem<N, NT, R, HT::LT>::BYTES;
   static std::atomic<unsigned long long> attr{0};
-  const size_t csmem = (size_t)COL_WARPS * COL_ARR * b->nzmax * sizeof(double);
+  const size_t csmem = (size_t)COL_WARPS * COL_ARR_MAX * b->nzmax * sizeof(double);
   auto limit = [](auto f, size_t bytes) {
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
@@ -2276,7 +2276,7 @@ void batch_enqueue_t(cgd_batch *b, WItem *const *w, bool p2alt)
     if constexpr (N == 5) limit(kb_phase2_flat<N, NT, R, P2_ALT_LEVELS>, FFA::SMEM);
 #endif
     for (auto f : {kb_column<0, C32>, kb_column<1, C32>, kb_column<2, C32>})
-      limit(f, COL_WARPS * COL_ARR * 64 * sizeof(double));
+      limit(f, COL_WARPS * COL_ARR_MAX * 64 * sizeof(double));
   }
   // (a list is empty when no member is of its kind)
   const int *n = b->n;
@@ -2382,7 +2382,7 @@ template <int NT, typename R>
 cudaError_t fused_setup_t(cgd_batch *b)
 {
   using CF = P2Cfg<5, NT, R, FUSED_P2_LEVELS>;
-  const size_t csm = (size_t)COL_WARPS * COL_ARR * b->nzmax * sizeof(double);
+  const size_t csm = (size_t)COL_WARPS * COL_ARR_MAX * b->nzmax * sizeof(double);
   b->fsmem = std::max(std::max(CF::SMEM, csm), HV1Smem<5, NT, R>::BYTES);
   static_assert(P2Flat<5, NT, R, FUSED_P2_LEVELS>::SMEM <= CF::SMEM, "the flat phase 2 needs no more");
   cudaError_t e = cudaFuncSetAttribute(kb_stage<5, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->fsmem);

@@ -72,6 +72,15 @@ __device__ __forceinline__ void cp_async4(float *smem_dst, const float *gsrc)
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// Ask for the bytes at p in L2 (whole 16-byte units, from the one p lies in)
+__device__ __forceinline__ void l2_prefetch(const void *p, size_t bytes)
+{
+  const size_t a = (size_t)p & ~(size_t)15, e = ((size_t)p + bytes) & ~(size_t)15;
+  if (e > a)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(__cvta_generic_to_global((const void *)a)),
+                 "r"((unsigned)(e - a)));
+}
+
 constexpr int NCOMP = 21;
 enum {
   C_D11_0 = 0, C_D11_1, C_D12_0, C_D12_1, C_D21_0, C_D21_1, C_D22_0, C_D22_1,
@@ -561,12 +570,16 @@ constexpr bool COL_KSUM = false;
 #endif
 
 constexpr int COL_WARPS = 8;
-// per warp: fv of rho, w, rho*theta, 8 bands, tri[3], x; each nz long.  (The
-// step's initial rho, w, rho*theta were once copied into three more arrays
-// by cp.async at the start for the update at the end; reading them at the
-// update instead is faster: 0.426/0.449 -> 0.411/0.427 ms for the second and
-// third stage on the drop-in grid, the smaller arrays leaving more L1.)
-constexpr int COL_ARR = 15;
+// Per warp: fv of rho, w, rho*theta and 8 bands, each nz long; tri[3] and x
+// take the rows of JWRho and JWRhoTh, which are dead by then, and the first
+// stage has two more rows.  (15 rows before: the second and third stage took
+// 0.368/0.362 ms instead of 0.353/0.345 on the drop-in grid, and at nz 64,
+// where only three CTAs fitted an SM, 1.45/1.42 instead of 1.24/1.18 ms on
+// nPanel 60.  Copying the step's initial rho, w, rho*theta into shared memory
+// at the start, for the update at the end, is slower than reading them there.)
+template <int MODE>
+constexpr int COL_ARR = MODE == 0 ? 13 : 11;
+constexpr int COL_ARR_MAX = COL_ARR<0>;
 // CTAs per SM the column kernel's registers are sized for: five for the first
 // stage (48 registers; 0.474 -> 0.464 ms on the drop-in grid), four for the
 // others (64 registers; five cost them 4-20 %)
@@ -742,6 +755,39 @@ __device__ __forceinline__ void stage_update(const ColArgs &A, size_t o, double 
   }
 }
 
+// A column's loads come in four rounds (table row, levels 0-31, 32-63, update)
+// that each wait for DRAM; the kernel moved 3.9 TB/s so.  Each warp therefore
+// starts with requests for all of its column's contributions, one row of nz
+// levels per lane, and the first warp for the CTA's columns of the states and
+// stage quantities, which lie side by side.  Column stages of one step, nPanel
+// 30, nz 45, NumTr 2: 0.387 + 0.415 + 0.384 -> 0.371 + 0.368 + 0.362 ms;
+// nPanel 60, nz 64: 1.86 + 1.83 + 1.73 -> 1.58 + 1.45 + 1.42 ms.  A launch of
+// less than one wave (four CTAs an SM) finds its data in L2: nPanel 6, nz 10
+// 14.5 -> 16.5 us with the requests.  (Plain prefetches of the second round's
+// and the update's lines: no gain; requests one wave ahead: slower, 0.50 ms.)
+constexpr int COL_PREFETCH_MIN = 4 * 148;
+
+template <int MODE, bool C32>
+__device__ __forceinline__ void column_prefetch(const GP &P, const ColArgs &A, int g0, int warp, int lane)
+{
+  const int nz = P.nz, NV = P.NV, g = g0 + warp;
+  const longlong2 *t = reinterpret_cast<const longlong2 *>(P.inv_tab) + 2 * (size_t)g;
+  const longlong2 ta = t[0], tb = t[1];
+  for (int r = lane; r < 4 * (NV + 1); r += 32) {
+    const int j = r & 3, f = r >> 2;
+    const long long off = j == 0 ? ta.x : j == 1 ? ta.y : j == 2 ? tb.x : tb.y;
+    const size_t es = C32 ? sizeof(float) : sizeof(double);
+    if (off >= 0) l2_prefetch(reinterpret_cast<const char *>(A.C) + (off + (size_t)f * P.DoF * nz) * es, nz * es);
+  }
+  if (warp > 0) return;
+  const int rows = NV * (MODE == 0 ? 1 : MODE == 2 && !COL_KSUM ? 3 : 2), cols = min(COL_WARPS, P.NumG - g0);
+  for (int r = lane; r < rows; r += 32) {
+    const int q = r / NV, f = r % NV;
+    const double *a = q == 0 ? A.Vn : q == 2 || (MODE == 2 && COL_KSUM) ? A.k2 : A.k1;
+    l2_prefetch(a + (size_t)nz * (g0 + (size_t)f * P.NumG), (size_t)cols * nz * sizeof(double));
+  }
+}
+
 template <int MODE, bool C32>
 __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const int bx)
 {
@@ -752,11 +798,12 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
   const int nz = P.nz, n = nz - 1, NV = P.NV, NumG = P.NumG;
   const bool valid = g < NumG;   // no early return: the block synchronises below
   const int LS = nz;                    // per-warp arrays of nz entries
-  double *sw = csm + (size_t)warp * COL_ARR * LS;
+  double *sw = csm + (size_t)warp * COL_ARR<MODE> * LS;
   double *fv = sw;                      // [3][nz]: rho, w, rho*theta
   double *jb = sw + 3 * LS;             // [8][nz]
-  double *tri = jb + 8 * LS;            // [3][nz]
-  double *xs = tri + 3 * LS;            // [nz]
+  double *tri = jb + 2 * LS;            // [3][nz], over JWRho, JWRhoTh
+  double *xs = jb + 5 * LS;             // [nz], over JWRhoTh
+  double *tmp = jb + 8 * LS;            // [2][nz], first stage
   const size_t fs = (size_t)nz * NumG;
   const double fac = A.fac;
   // k1, k2 of the Schur fields (rho, w, rho*theta), kept for the update
@@ -775,6 +822,8 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
       for (int r = 0; r < 8; ++r) cp_async8(jb + r * LS + l, jg + r * js);
     }
   }
+
+  if (MODE <= 2 && valid && gridDim.x >= COL_PREFETCH_MIN) column_prefetch<MODE, C32>(P, A, g0, warp, lane);
 
   // 1. tendency (owner gather) + stage corrections; fields outside the Schur
   //    system finished here; bands
@@ -830,10 +879,10 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
         // dPresdRhoTh once per level, shared with the interface below
 #ifdef CGD_FAST
         // Rd (Rd rhotheta / p0)^(kappa/(1-kappa)) = p / rhotheta with the pressure at hand
-        xs[l] = A.ps[o0] / A.Vn[o0 + 4 * fs];
-        tri[l] = 1.0 / P.dz[o0];
+        tmp[l] = A.ps[o0] / A.Vn[o0 + 4 * fs];
+        tmp[LS + l] = 1.0 / P.dz[o0];
 #else
-        xs[l] = dpdrhoth(P, A.Vn[o0 + 4 * fs]);
+        tmp[l] = dpdrhoth(P, A.Vn[o0 + 4 * fs]);
 #endif
       }
     } else {
@@ -861,10 +910,10 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
         double b[8];
         const double *V0 = A.Vn + (size_t)nz * g;
 #ifdef CGD_FAST
-        jac_bands_rcp(P, V0[l], V0[l + 1], V0[l + 4 * fs], V0[l + 1 + 4 * fs], xs[l], xs[l + 1],
-                      P.dz[l + (size_t)nz * g], P.dz[l + 1 + (size_t)nz * g], tri[l], tri[l + 1], b);
+        jac_bands_rcp(P, V0[l], V0[l + 1], V0[l + 4 * fs], V0[l + 1 + 4 * fs], tmp[l], tmp[l + 1],
+                      P.dz[l + (size_t)nz * g], P.dz[l + 1 + (size_t)nz * g], tmp[LS + l], tmp[LS + l + 1], b);
 #else
-        jac_bands(P, V0[l], V0[l + 1], V0[l + 4 * fs], V0[l + 1 + 4 * fs], xs[l], xs[l + 1],
+        jac_bands(P, V0[l], V0[l + 1], V0[l + 4 * fs], V0[l + 1 + 4 * fs], tmp[l], tmp[l + 1],
                   P.dz[l + (size_t)nz * g], P.dz[l + 1 + (size_t)nz * g], b);
 #endif
 #pragma unroll
@@ -882,7 +931,7 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
 #define FV3(i) fv[LS + (i)]
 #define FV4(i) fv[2 * LS + (i)]
   const double invfac2 = A.ifac2;
-  double v3new[2] = {0.0, 0.0};
+  double v3new[2] = {0.0, 0.0}, tq[2][3];
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
     const int l = lane + 32 * it;
@@ -894,7 +943,7 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
       else t0 = -JB(1, 0, l - 1) * JB(0, 0, l) - JB(2, 0, l - 1) * JB(3, 0, l);
       if (l == n - 1) t2 = 0.0;
       else t2 = -JB(1, 1, l + 1) * JB(0, 1, l) - JB(2, 1, l + 1) * JB(3, 1, l);
-      tri[l] = t0; tri[LS + l] = t1; tri[2 * LS + l] = t2;
+      tq[it][0] = t0; tq[it][1] = t1; tq[it][2] = t2;
       // SchurSolveFKernel!
 #ifdef CGD_FAST
       const double v3 = FV3(l) * A.ifac;
@@ -908,7 +957,11 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
   __syncwarp();
 #pragma unroll
   for (int it = 0; it < 2; ++it)
-    if (valid && lane + 32 * it < n) FV3(lane + 32 * it) = v3new[it];
+    if (valid && lane + 32 * it < n) {
+      FV3(lane + 32 * it) = v3new[it];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) tri[r * LS + lane + 32 * it] = tq[it][r];
+    }
 #ifdef CGD_FAST
   // triSolve! as three warp scans over the column's levels (fast build);
   // the result differs from the sequential sweep by rounding only
@@ -921,10 +974,10 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
   // triSolve! (Thomas), b = FV3, x = xs: the serial sweeps of the block's
   // columns run concurrently, one per lane of the first warp
   if (threadIdx.x < COL_WARPS && g0 + (int)threadIdx.x < NumG) {
-    double *sc = csm + (size_t)threadIdx.x * COL_ARR * LS;
+    double *sc = csm + (size_t)threadIdx.x * COL_ARR<MODE> * LS;
     double *b = sc + LS;
-    const double *tr = sc + 11 * LS;
-    double *x = sc + 14 * LS;
+    const double *tr = sc + 5 * LS;
+    double *x = sc + 8 * LS;
     x[0] = tr[LS + 0];
     for (int i = 0; i < n - 1; ++i) {
       const double m = tr[2 * LS + i] / x[i];   // the reference's tri[3,i]/x[i], used twice
