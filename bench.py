@@ -269,6 +269,13 @@ def step_bytes(cfg):
     return tot + 3 * S + 8 * Sp + 5 * NV * S
 
 
+def step_launches(nf, p, nz):
+    """Kernel launches of one captured step of nf elements: phase 1, phase 2
+    and the column kernel in three stages; phase 2 is two launches from 4096
+    CTAs a role on (one per element and 16 levels, 32 at p = 1)."""
+    return 3 * (3 if nf * -(-nz // (32 if p == 1 else 16)) < 4096 else 4)
+
+
 def ncu_traffic():
     """Per-launch DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of
     the phase-2 kernel from the committed ncu summary of the drop-in workload."""
@@ -635,7 +642,7 @@ def ensemble_measure(K, warmup, rank, ranks, torch):
             "mass_drift_fp64_max": float(max(abs(x) for x in res["fp64"]["drift"])),
             "finite": res["fp64"]["finite"] and res["mixed"]["finite"],
             "perturbation": f"theta +-{E['theta_amp']} K, u,v +-{E['wind_amp']} m/s, seed {E['seed0']}+member",
-            "gpu_launches": {"fused": 3, "members": 9 * len(members)}.get(
+            "gpu_launches": {"fused": 3, "members": sum(step_launches(m[0].NF, 4, m[0].nz) for m in members)}.get(
                 res["fp64"]["tuning"].split("stage=")[1].split(";")[0], 9) * K}
 
 
@@ -836,7 +843,7 @@ def run_ours(args, cfg, rank, world, local):
             "adjoint": adjoint,
             "ensemble": ensemble,
             "output": outp,
-            "gpu_launches": 9 * args.steps,
+            "gpu_launches": step_launches(6 * cfg.nPanel ** 2, cfg.OrdPoly, cfg.nz) * args.steps,
             "cpu_baseline": cpu,
             "clocks": clk,
         }
@@ -912,7 +919,7 @@ def run_shard(args, cfg, rank, world, local):
                 "e2e": {"value": Ke / te, "unit": UNIT, "h2d_bytes_per_step": tot_bytes,
                         "d2h_bytes_per_step": tot_bytes, "steps": Ke,
                         "call": "cgd_ros_step(h_rank, host_part, dt, 1) per step on every rank"},
-                "gpu_launches": (9 + (12 if world > 1 else 0)) * args.steps, "clocks": clk}
+                "gpu_launches": (step_launches(6 * cfg.nPanel ** 2 // world, cfg.OrdPoly, cfg.nz) + (12 if world > 1 else 0)) * args.steps, "clocks": clk}
         print(json.dumps(line), flush=True)
     d.close()
     if world > 1:

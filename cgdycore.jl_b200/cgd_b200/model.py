@@ -506,7 +506,7 @@ class PartGroup:
 class Ensemble:
     """Batched ensemble of Dycore members (same OrdPoly, NumTr and precision;
     any nPanel and nz): one ensemble step is one CUDA graph over flat work
-    lists spanning every member (cgd_batch_step), either 15 launches or, with
+    lists spanning every member (cgd_batch_step), either 9 launches or, with
     fused=True (OrdPoly 4), one persistent cooperative launch per stage; or,
     with members=True, one graph branch per member running that member's own
     step.  autotune=True times every work-list order in every form and keeps

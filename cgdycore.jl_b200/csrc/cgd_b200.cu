@@ -269,9 +269,18 @@ void launch_p2r(cgd_handle *h, const double *U, const double *Pr, const double *
   if (gp.flat) {
     using FF = P2Flat<N, NT, R>;
     static std::atomic<unsigned long long> fattr{0};
-    if (first_on_device(fattr))
+    if (first_on_device(fattr)) {
       cudaFuncSetAttribute(k_phase2_flat<N, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FF::SMEM);
-    k_phase2_flat<N, NT, R><<<grid, FF::THREADS, FF::SMEM, h->stream>>>(gp, U, Pr, C1, C);
+      cudaFuncSetAttribute(k_phase2_momentum<N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FF::M_BYTES);
+      cudaFuncSetAttribute(k_phase2_scalars<N, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FF::S_BYTES);
+    }
+    const dim3 half(grid.x / 2, grid.y);
+    if ((long long)half.x * half.y < P2_SPLIT_MIN) {
+      k_phase2_flat<N, NT, R><<<grid, FF::THREADS, FF::SMEM, h->stream>>>(gp, U, Pr, C1, C);
+    } else {
+      k_phase2_momentum<N, R><<<half, FF::THREADS, FF::M_BYTES, h->stream>>>(gp, U, Pr, C1, C);
+      k_phase2_scalars<N, NT, R><<<half, FF::THREADS, FF::S_BYTES, h->stream>>>(gp, U, C1, C);
+    }
     return;
   }
 #endif
@@ -898,20 +907,8 @@ static int create_impl(const cgd_config *cfg, const int64_t *glob, const double 
     if (ptr[g + 1] - ptr[g] <= 4)
       for (int q = ptr[g]; q < ptr[g + 1]; ++q) tab[(size_t)4 * g + (q - ptr[g])] = off[q];
   TRY(dalloc(h, &h->inv_tab, tab.size()));
-  // the same rows per element node (offsets in units of nz), and the first
-  // local contributor of every DOF (it writes the DOF's pressure)
-  std::vector<int4> etab((size_t)DoF * NF);
-  std::vector<unsigned char> own((size_t)DoF * NF, 0);
-  std::vector<unsigned char> seen(NumG, 0);
-  for (size_t i = 0; i < etab.size(); ++i) {
-    const int g = glob0[i];
-    const long long *r = &tab[(size_t)4 * g];
-    auto at = [&](int k) { return r[k] < 0 ? -1 : (int)(r[k] / nz); };
-    etab[i] = int4{at(0), at(1), at(2), at(3)};
-    if (!seen[g]) own[i] = seen[g] = 1;
-  }
-  TRY(dalloc(h, &h->etab, etab.size()));
-  TRY(dalloc(h, &h->own, own.size()));
+  TRY(dalloc(h, &h->etab, glob0.size()));
+  TRY(dalloc(h, &h->own, glob0.size()));
   // contribution buffer: the local elements, then the ghost pseudo-elements
   const size_t ghost_elems = ((size_t)nghost + DoF - 1) / DoF;
   TRY(dalloc(h, &h->C, ENL * (NV + 1) + ghost_elems * DoF * nz * (NV + 1)));
@@ -947,25 +944,24 @@ static int create_impl(const cgd_config *cfg, const int64_t *glob, const double 
   if ((!dev_metric && up(h->met, met.data(), met.size() * 8)) || cudaGetLastError() != cudaSuccess || up(h->M, M, 2 * S * 8) || up(h->dz, dz, S * 8) ||
       up(h->glob, glob0.data(), glob0.size() * 4) || up(h->inv_ptr, ptr.data(), ptr.size() * 4) ||
       up(h->inv_off, off.data(), off.size() * 8) || up(h->inv_tab, tab.data(), tab.size() * 8) ||
-      up(h->etab, etab.data(), etab.size() * sizeof(int4)) || up(h->own, own.data(), own.size()) ||
       (halo && nsend && up(h->send_list, halo->send_list, (size_t)nsend * 4))) {
     cudaError_t e = cudaGetLastError();
     cuda_fail(h, e, "cgd_create upload");
     cgd_destroy(h);
     return CGD_ERR_CUDA;
   }
-  if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
-    cuda_fail(h, cudaGetLastError(), "cgd_create sync");
-    cgd_destroy(h);
-    return CGD_ERR_CUDA;
-  }
-
   h->glob_host = glob0;
   GP &P = h->gp;
   P.N = N; P.DoF = DoF; P.nz = nz; P.NF = NF; P.NumG = NumG; P.NumTr = h->NumTr; P.NV = NV; P.NC = NV + 1;
   P.met = h->met; P.M = h->M; P.dz = h->dz; P.glob = h->glob; P.inv_ptr = h->inv_ptr; P.inv_off = h->inv_off;
   P.inv_tab = h->inv_tab; P.etab = h->etab; P.own = h->own;
   P.pref = h->pref; P.thref = h->thref;
+  k_node_tables<<<(unsigned)((glob0.size() + 255) / 256), 256, 0, h->stream>>>(P, h->etab, h->own);
+  if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
+    cuda_fail(h, cudaGetLastError(), "cgd_create sync");
+    cgd_destroy(h);
+    return CGD_ERR_CUDA;
+  }
   for (int i = 0; i < 25; ++i) { P.D[i] = 0.0; P.DW[i] = 0.0; }
   for (int i = 0; i < N * N; ++i) { P.D[i] = DS[i]; P.DW[i] = DW[i]; }
   P.Grav = cfg->Grav; P.Rd = cfg->Rd; P.p0 = cfg->p0; P.kappa = cfg->Rd / cfg->Cpd;

@@ -9,9 +9,9 @@
 // 9 launches, whatever the number of members.
 //
 // The fused form (kb_stage, p = 4) runs a whole stage - phase 1 with the
-// pressure, phase 2, the column solve and update - as one persistent cooperative launch whose CTAs walk the same work lists,
-// with a grid barrier between the parts: one ensemble step is three
-// launches.  Within one launch no array is read, rewritten and read again
+// pressure, phase 2, the column solve and update - as one persistent
+// cooperative launch whose CTAs walk the same work lists, with a grid barrier
+// between the parts: one ensemble step is three launches.  Within one launch no array is read, rewritten and read again
 // (the phases write contribution buffers of their own, the stage-3 state goes to
 // a second stage buffer Vst2), so no CTA can read a line that an earlier part
 // of the same launch left in its caches before another CTA rewrote it.

@@ -295,7 +295,7 @@ struct P2Flat {
   static constexpr int M_PLANES = 4 + 2 + 2 + 2;
   static constexpr size_t M_BYTES = ((size_t)2 * RS + (size_t)M_PLANES * PL + (size_t)4 * (PL + RS)) * sizeof(R);
   static constexpr size_t SMEM = S_BYTES > M_BYTES ? S_BYTES : M_BYTES;
-  static constexpr int MINB = G::MINB;
+  static constexpr int MINB = G::MINB, MINB_S = 1280 / THREADS;
 };
 
 template <int N, int NT, typename R, int LT, int TH>
@@ -697,6 +697,36 @@ __global__ void __launch_bounds__(P2Flat<N, NT, R>::THREADS, P2Flat<N, NT, R>::M
                   const double *__restrict__ C1, double *__restrict__ C)
 {
   phase2_flat<N, NT, R>(P, U, Pr, C1, C, blockIdx.x, launch_element(P));
+}
+
+// The roles in launches of their own: the scalars' needs fewer registers, so
+// that half as many CTAs again fit an SM (48 registers; at p = 4 three CTAs
+// instead of two), which one launch of both cannot use.  From P2_SPLIT_MIN CTAs
+// of each role on (some 14 waves of the momentum role).  One launch -> two, ms:
+// nPanel 60, nz 64 3.37 -> 3.16 (86400 CTAs); nPanel 30, nz 45, two tracers
+// 0.790 -> 0.784 (16200); nPanel 30, p 3, nz 31 0.270 -> 0.261 (10800); below,
+// the second launch's tail and start cost more: nPanel 16, nz 30 0.1305 ->
+// 0.1321 (3072), nPanel 6, nz 10 0.018 -> 0.021 (216).  The momentum role at 48
+// registers spills and takes longer (0.89 for 0.79 together).
+constexpr int P2_SPLIT_MIN = 4096;
+
+template <int N, typename R>
+__global__ void __launch_bounds__(P2Flat<N, 0, R>::THREADS, P2Flat<N, 0, R>::MINB)
+    k_phase2_momentum(const GP P, const double *__restrict__ U, const double *__restrict__ Pr,
+                      const double *__restrict__ C1, double *__restrict__ C)
+{
+  extern __shared__ double sm[];
+  using F = P2Flat<N, 0, R>;   // (the role is the same with tracers)
+  phase2_momentum_flat<N, 0, R, F::LT, F::THREADS>(P, U, Pr, C1, C, blockIdx.x * F::LT, launch_element(P), sm);
+}
+
+template <int N, int NT, typename R>
+__global__ void __launch_bounds__(P2Flat<N, NT, R>::THREADS, P2Flat<N, NT, R>::MINB_S)
+    k_phase2_scalars(const GP P, const double *__restrict__ U, const double *__restrict__ C1, double *__restrict__ C)
+{
+  extern __shared__ double sm[];
+  using F = P2Flat<N, NT, R>;
+  phase2_scalars_flat<N, NT, R, F::LT, F::THREADS>(P, U, C1, C, blockIdx.x * F::LT, launch_element(P), sm);
 }
 
 }  // namespace cgd

@@ -206,4 +206,20 @@ __global__ void __launch_bounds__(256) k_compact_metric(int DoF, int nz, int NF,
   for (int c = 0; c < NCOMP; ++c) met[(((size_t)IF * NCOMP + c) * DoF + ID) * nz + Iz] = v[c];
 }
 
+// Per element node: its DOF's inv_tab row in units of nz, and whether it is the
+// DOF's first local contributor (ghost contributions lie behind the elements').
+__global__ void __launch_bounds__(256) k_node_tables(const GP P, int4 *__restrict__ etab, unsigned char *__restrict__ own)
+{
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= P.DoF * P.NF) return;
+  const int g = P.glob[i];
+  const long long *r = P.inv_tab + 4 * (size_t)g;
+  auto at = [&](int k) { return r[k] < 0 ? -1 : (int)(r[k] / P.nz); };
+  etab[i] = int4{at(0), at(1), at(2), at(3)};
+  const long long me = ((long long)(i / P.DoF) * P.NC * P.DoF + i % P.DoF) * P.nz;
+  bool first = true;
+  for (int q = P.inv_ptr[g]; q < P.inv_ptr[g + 1]; ++q) first = first && P.inv_off[q] >= me;
+  own[i] = first;
+}
+
 }  // namespace cgd

@@ -372,7 +372,7 @@ int cgd_jac_schur_solve_noalloc(const cgd_config *cfg, const double *U, const do
  * ensemble step advances every member by one Rosenbrock-W step of its own
  * dt, as one CUDA graph over flat work lists spanning all members (the
  * kernels of one stage read each member's parameters from constant memory):
- * either 15 launches (split form) or, with CGD_BATCH_FUSED (OrdPoly 4 only,
+ * either 9 launches (split form) or, with CGD_BATCH_FUSED (OrdPoly 4 only,
  * CGD_ERR_UNSUPPORTED otherwise), three persistent cooperative launches, one
  * per stage, each running pressure, both tendency phases with their DSS and
  * the column solve and update with a grid barrier between them (fused form;
