@@ -1150,7 +1150,7 @@ int cgd_jac_bands(cgd_handle *h, const double *U, double *JRhoW, double *JWRho, 
   const size_t bytes = (size_t)2 * (h->nz - 1) * h->NumG * 8;
   Bands4 direct{};
   for (int i = 0; i < 4; ++i) {
-    bool apart = dev[i] && on_this_device(user[i]) && (uintptr_t)user[i] % sizeof(double) == 0 &&
+    bool apart = dev[i] && on_this_device(user[i]) && (uintptr_t)user[i] % sizeof(double2) == 0 &&
                  !overlaps(user[i], bytes, Ud, (size_t)h->nz * h->NumG * h->NV * 8) &&
                  !overlaps(user[i], bytes, h->bands, 4 * bytes);
     for (int j = 0; j < 4; ++j) apart = apart && (j == i || !overlaps(user[i], bytes, user[j], bytes));

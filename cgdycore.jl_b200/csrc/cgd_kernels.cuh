@@ -1106,9 +1106,10 @@ __global__ void __launch_bounds__(256) k_physics(const GP P, const double *__res
 
 // Jacobian bands into memory (cgd_jac): one thread per (level, column), which
 // evaluates dp/d(rho theta) of its level and takes the upper level's from the
-// next thread, and writes the bands of the interface above; out2 (null
-// entries: none) takes a copy for the caller.  nPanel 20, nz 37: 47 us and four
-// copies of the bands before.
+// next thread, and writes the bands of the interface above, a pair (16 bytes)
+// per store; out2 (null entries: none) takes a copy for the caller.  nPanel 20,
+// nz 37: 47 us and four copies of the bands before; now 64 us for
+// all (70 us with single stores).
 __global__ void __launch_bounds__(256) k_jac(const GP P, const double *__restrict__ U, const Bands4 out,
                                              const Bands4 out2)
 {
@@ -1125,14 +1126,13 @@ __global__ void __launch_bounds__(256) k_jac(const GP P, const double *__restric
   if (l == n) return;
   double b[8];
   jac_bands(P, U[tid], U[tid + 1], U[tid + 4 * S], U[tid + 1 + 4 * S], dp[t], dp[t + 1], P.dz[tid], P.dz[tid + 1], b);
-  const size_t o = 2 * (l + (size_t)n * g);
+  const size_t o = l + (size_t)n * g;
 #pragma unroll
-  for (int arr = 0; arr < 4; ++arr)
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      out.b[arr][o + r] = b[arr * 2 + r];
-      if (out2.b[arr]) out2.b[arr][o + r] = b[arr * 2 + r];
-    }
+  for (int arr = 0; arr < 4; ++arr) {
+    const double2 b2 = {b[2 * arr], b[2 * arr + 1]};
+    reinterpret_cast<double2 *>(out.b[arr])[o] = b2;
+    if (out2.b[arr]) reinterpret_cast<double2 *>(out2.b[arr])[o] = b2;
+  }
 }
 
 __device__ __forceinline__ void pressure_body(const GP &P, const double *__restrict__ U, double *__restrict__ p,
