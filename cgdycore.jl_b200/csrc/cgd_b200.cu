@@ -65,6 +65,7 @@ struct cgd_handle {
   std::vector<Buf> bufs;
   double *met = nullptr, *M = nullptr, *dz = nullptr;
   double *hm = nullptr, *zl = nullptr;   // factors of a flat product grid (GP::hm, GP::zl)
+  unsigned form = 0;   // counts the changes of the kernels' form (GP::flat, the factors); an ensemble compares it
   int *glob = nullptr, *inv_ptr = nullptr;
   int4 *etab = nullptr;
   unsigned char *own = nullptr;
@@ -1416,10 +1417,14 @@ int cgd_set_layers(cgd_handle *h, const double *z)
   for (int l = 0; l < h->nz; ++l)
     if (!(z[l] > 0.0)) return CGD_ERR_INVALID_ARG;
 #ifdef CGD_FAST
-  if (int rc = flat_factors(h, z)) return rc;
+  if (int rc = enter(h)) return rc;
+  const int rc = flat_factors(h, z);
   free_graph(h);
-#endif
+  ++h->form;
+  return rc;
+#else
   return CGD_OK;
+#endif
 }
 
 int cgd_set_exchange(cgd_handle *h, cgd_exchange_fn fn, void *user)
@@ -2133,6 +2138,7 @@ struct cgd_batch {
   GridBar *bar = nullptr;
   std::vector<double *> Vst2;
   std::vector<GP> gps;
+  std::vector<unsigned> form;   // cgd_handle::form of the members that gps and the work lists are of
   std::vector<BMember> bms;
   std::vector<void *> scratch;
   // the members form: fork and join events, and the states and time steps
@@ -2456,6 +2462,43 @@ int fused_timed_out(cgd_batch *b)
   return t != 0;
 }
 
+// The members' parameters and the work lists of every order in use; graphs and
+// tuning of earlier ones are dropped.
+int batch_members(cgd_batch *b)
+{
+  for (int c = 0; c < cgd_batch::NCAND; ++c) {
+    if (b->gexec[c]) cudaGraphExecDestroy(b->gexec[c]);
+    if (b->graph[c]) cudaGraphDestroy(b->graph[c]);
+    b->gexec[c] = nullptr;
+    b->graph[c] = nullptr;
+  }
+  b->tuned = false;
+  b->form.clear();
+  b->gps.clear();
+  std::vector<unsigned> form;
+  for (const cgd_handle *h : b->mem) {
+    b->gps.push_back(h->gp);
+    form.push_back(h->form);
+  }
+  const int nord = b->autotune ? cgd_batch::NORD : 1;
+  for (int o = 0; o < nord; ++o) {
+    std::vector<WItem> lists[WL_N];
+    batch_lists(b, o, lists);
+    for (int k = 0; k < WL_N; ++k) {
+      if (b->w[o][k]) cudaFree(b->w[o][k]);
+      b->w[o][k] = nullptr;
+      b->n[k] = (int)lists[k].size();
+      if (lists[k].empty()) continue;
+      void *p = nullptr;
+      BCK(cudaMalloc(&p, lists[k].size() * sizeof(WItem)));
+      b->w[o][k] = static_cast<WItem *>(p);
+      BCK(cudaMemcpy(p, lists[k].data(), lists[k].size() * sizeof(WItem), cudaMemcpyHostToDevice));
+    }
+  }
+  b->form = form;   // set last: a failure above is tried again by the next step
+  return CGD_OK;
+}
+
 int batch_upload(cgd_batch *b)
 {
   const size_t nm = b->mem.size();
@@ -2542,26 +2585,10 @@ int cgd_batch_create(cgd_handle *const *members, int32_t nmembers, int32_t flags
       }
       if (e != cudaSuccess) { rc = batch_fail(b, e, "cgd_batch_create fused buffers"); break; }
     }
-    const int nord = b->autotune ? cgd_batch::NORD : 1;
-    for (int o = 0; o < nord && !rc; ++o) {
-      std::vector<WItem> lists[WL_N];
-      batch_lists(b, o, lists);
-      for (int k = 0; k < WL_N; ++k) {
-        b->n[k] = (int)lists[k].size();
-        void *p = nullptr;
-        if (lists[k].empty()) continue;
-        e = cudaMalloc(&p, lists[k].size() * sizeof(WItem));
-        if (e == cudaSuccess)
-          e = cudaMemcpy(p, lists[k].data(), lists[k].size() * sizeof(WItem), cudaMemcpyHostToDevice);
-        b->w[o][k] = static_cast<WItem *>(p);
-        if (e != cudaSuccess) { rc = batch_fail(b, e, "cgd_batch_create work lists"); break; }
-      }
-    }
+    rc = batch_members(b);
   } while (false);
   if (rc) { cgd_batch_destroy(b); return rc; }
-  b->gps.resize(nmembers);
   b->bms.resize(nmembers);
-  for (int m = 0; m < nmembers; ++m) b->gps[m] = members[m]->gp;
   *out = b;
   return CGD_OK;
 }
@@ -2599,6 +2626,14 @@ int cgd_batch_step(cgd_batch *b, double *const *U, const double *dt, int32_t nst
   BCK(cudaSetDevice(b->device));
   BCK(cudaEventRecord(b->order_ev, b->mem[0]->caller));
   BCK(cudaStreamWaitEvent(b->stream, b->order_ev, 0));
+  // a member that changed its kernels' form since (cgd_set_layers): the copies
+  // of its parameters, the lists and the captured launches are of the old one
+  bool changed = b->form.size() != b->mem.size();
+  for (int m = 0; m < nm && !changed; ++m) changed = b->form[m] != b->mem[m]->form;
+  if (changed) {
+    BCK(cudaStreamSynchronize(b->stream));
+    if (int rc = batch_members(b)) return rc;
+  }
   // mixed members: the reference profile from their first state
   for (int m = 0; m < nm; ++m) {
     cgd_handle *h = b->mem[m];

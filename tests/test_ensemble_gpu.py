@@ -113,3 +113,36 @@ def test_grid_barrier_holds_and_times_out(built_lib, cuda_ok):
     assert time.perf_counter() - t0 < 5.0
     assert L.cgd_grid_barrier_check(50, 0, 2.0, ctypes.byref(v)) == 0
     assert v.value == 0
+
+
+@pytest.mark.parametrize("form", ["split", "fused", "members", "autotune"])
+def test_member_changes_its_layers(oracle_mod, built_lib, cuda_ok, form):
+    """Layer ratios given to a member after the ensemble was made (and
+    stepped): wrong ones send the member to the general kernels, the right
+    ones back to the flat ones, as when it is stepped on its own; the other
+    members keep theirs."""
+    from cgd_b200 import Ensemble, _lib
+    from cgd_b200.grid import layer_ratios
+
+    def set_layers(d, z):
+        z = np.ascontiguousarray(z)
+        _lib.check(d._L.cgd_set_layers(d.h, z.ctypes.data), "cgd_set_layers")
+
+    mem, alone = _members(oracle_mod, False), _members(oracle_mod, False)
+    dts = [dt for _, _, dt in mem]
+    ens = Ensemble([d for d, _, _ in mem], autotune=form == "autotune", fused=form == "fused",
+                   members_form=form == "members")
+    states, ref = [_dev(U) for _, U, _ in mem], [_dev(U) for _, U, _ in alone]
+    right = layer_ratios(alone[1][0].grid)
+    for z in (None, right * 1.01 ** np.arange(right.size), right):
+        if z is not None:
+            set_layers(mem[1][0], z)
+            set_layers(alone[1][0], z)
+        ens.step(states, dts, 1)
+        for (d, _, dt), V in zip(alone, ref):
+            d.time_stepper(V, dt, 1)
+        for s, V in zip(states, ref):
+            assert np.array_equal(_host(s), _host(V))
+    ens.close()
+    for d, _, _ in mem + alone:
+        d.close()
