@@ -33,7 +33,7 @@ EXPORTS = [
     "cgd_tape_record_step", "cgd_tape_step_adjoint", "cgd_tape_release", "cgd_tape_bytes_per_step",
     "cgd_batch_create", "cgd_batch_step", "cgd_batch_tuning", "cgd_batch_get_stream", "cgd_batch_destroy",
     "cgd_grid_barrier_check",
-    "cgd_create_part", "cgd_set_layers", "cgd_set_exchange", "cgd_halo_buffers", "cgd_group_rhs", "cgd_group_ros_step",
+    "cgd_create_part", "cgd_set_layers", "cgd_flat_form", "cgd_set_flat_form", "cgd_set_exchange", "cgd_halo_buffers", "cgd_group_rhs", "cgd_group_ros_step",
     "cgd_metric_sphere", "cgd_mass_dz", "cgd_set_physics",
     "cgd_vtk_inter", "cgd_interpolate", "cgd_interpolate_wb", "cgd_interpolate_vort", "cgd_output_fields",
 ]
@@ -111,6 +111,10 @@ def lib(exact=False):
         L.cgd_create_part.restype = ctypes.c_int
         L.cgd_set_layers.argtypes = [vp, vp]
         L.cgd_set_layers.restype = ctypes.c_int
+        L.cgd_flat_form.argtypes = [vp, ctypes.POINTER(ctypes.c_int32)]
+        L.cgd_flat_form.restype = ctypes.c_int
+        L.cgd_set_flat_form.argtypes = [vp, ctypes.c_int32]
+        L.cgd_set_flat_form.restype = ctypes.c_int
         L.cgd_set_exchange.argtypes = [vp, EXCHANGE_FN, vp]
         L.cgd_set_exchange.restype = ctypes.c_int
         L.cgd_halo_buffers.argtypes = [vp, ctypes.POINTER(vp), ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(vp),

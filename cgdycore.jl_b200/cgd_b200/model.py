@@ -159,12 +159,25 @@ class Dycore:
         xp = X.data_ptr() if hasattr(X, "data_ptr") else np.asfortranarray(X).ctypes.data
         _lib.check(self._L.cgd_set_physics(self.h, ctypes.byref(ph), xp), "cgd_set_physics")
 
+    def flat_form(self):
+        """Whether the handle runs the flat-grid kernels (cgd_flat_form)."""
+        f = ctypes.c_int32()
+        _lib.check(self._L.cgd_flat_form(self.h, ctypes.byref(f)), "cgd_flat_form")
+        return bool(f.value)
+
+    def set_flat_form(self, on):
+        """Refuse the flat-grid kernels, or let the grid's check decide again."""
+        _lib.check(self._L.cgd_set_flat_form(self.h, int(bool(on))), "cgd_set_flat_form")
+
     def set_transport(self, transport):
         """The exchange of a decomposed grid's rank between processes:
         transport.exchange(send_views, recv_views) (parallel.TorchTransport)
         is called at every DSS point with device views of the library's
-        packed buffers, on the library's stream."""
+        packed buffers, on the library's stream.  A transport with all_flat
+        makes the ranks agree on the kernels' form, so every rank calls this."""
         import torch
+        if hasattr(transport, "all_flat"):
+            self.set_flat_form(transport.all_flat(self.flat_form()))
         P = self.halo
         sp, sn, rp, rn = ctypes.c_void_p(), ctypes.c_int64(), ctypes.c_void_p(), ctypes.c_int64()
         _lib.check(self._L.cgd_halo_buffers(self.h, ctypes.byref(sp), ctypes.byref(sn), ctypes.byref(rp),

@@ -207,6 +207,19 @@ class TorchTransport:
         self.plan = plan
         self.group = group
 
+    def all_flat(self, flat):
+        """Whether `flat` holds on every rank (a collective of the group): one
+        rank with an element that is not of the flat form sends all to the
+        general kernels, as on the whole grid."""
+        import torch
+        import torch.distributed as dist
+        if not dist.is_initialized():
+            return bool(flat)
+        dev = "cuda" if dist.get_backend(self.group) == "nccl" else "cpu"
+        t = torch.tensor([int(bool(flat))], device=dev)
+        dist.all_reduce(t, op=dist.ReduceOp.MIN, group=self.group)
+        return bool(t.item())
+
     def exchange(self, send_views, recv_views):
         """send_views[i] goes to plan.neighbours[i], recv_views[i] is filled
         from it."""

@@ -65,6 +65,9 @@ struct cgd_handle {
   std::vector<Buf> bufs;
   double *met = nullptr, *M = nullptr, *dz = nullptr;
   double *hm = nullptr, *zl = nullptr;   // factors of a flat product grid (GP::hm, GP::zl)
+  // GP::flat follows from three things (choose_form): this grid's check, the
+  // caller's consent, and on a part of a decomposed grid the whole grid's layers
+  bool flat_ok = false, flat_on = true, layers = false;
   unsigned form = 0;   // counts the changes of the kernels' form (GP::flat, the factors); an ensemble compares it
   int *glob = nullptr, *inv_ptr = nullptr;
   int4 *etab = nullptr;
@@ -651,7 +654,7 @@ int flat_factors(cgd_handle *h, const double *zin)
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(&bad, h->flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  P.flat = !bad;
+  h->flat_ok = !bad;
   return CGD_OK;
 }
 #endif
@@ -663,6 +666,17 @@ void free_graph(cgd_handle *h)
   h->gexec = nullptr;
   h->graph = nullptr;
   h->graph_U = nullptr;
+}
+
+// The kernels the handle runs from now on.  Flat and general kernels round
+// differently, so the parts of a decomposed grid must all run the same, with the
+// same layers, to agree with one another: a part that was not given the whole
+// grid's layers runs the general ones.
+void choose_form(cgd_handle *h)
+{
+  h->gp.flat = h->flat_ok && h->flat_on && (!h->decomposed || h->layers);
+  free_graph(h);
+  ++h->form;
 }
 
 int check_cfg(const cgd_config *c)
@@ -977,6 +991,7 @@ static int create_impl(const cgd_config *cfg, const int64_t *glob, const double 
     P.hm = h->hm = hm;
     P.zl = h->zl = hm + nh;
     TRY(flat_factors(h, nullptr));
+    choose_form(h);
   }
 #endif
 
@@ -1418,13 +1433,31 @@ int cgd_set_layers(cgd_handle *h, const double *z)
     if (!(z[l] > 0.0)) return CGD_ERR_INVALID_ARG;
 #ifdef CGD_FAST
   if (int rc = enter(h)) return rc;
+  h->flat_ok = false;
   const int rc = flat_factors(h, z);
-  free_graph(h);
-  ++h->form;
+  h->layers = rc == CGD_OK;
+  choose_form(h);
   return rc;
 #else
   return CGD_OK;
 #endif
+}
+
+int cgd_flat_form(cgd_handle *h, int32_t *flat)
+{
+  if (!h || !flat) return CGD_ERR_INVALID_ARG;
+  *flat = h->gp.flat;
+  return CGD_OK;
+}
+
+int cgd_set_flat_form(cgd_handle *h, int32_t on)
+{
+  if (!h) return CGD_ERR_INVALID_ARG;
+  if (h->flat_on != (on != 0)) {
+    h->flat_on = on != 0;
+    choose_form(h);
+  }
+  return CGD_OK;
 }
 
 int cgd_set_exchange(cgd_handle *h, cgd_exchange_fn fn, void *user)
@@ -1446,8 +1479,13 @@ int cgd_halo_buffers(cgd_handle *h, double **send, int64_t *send_doubles, double
 }
 
 // Checks of an in-process group: parts[r] is rank r, one device, ranks and
-// exchange sizes consistent.  The parts then run on parts[0]'s stream.
-static int group_enter(cgd_handle *const *parts, int32_t n, std::vector<cudaStream_t> &saved)
+// exchange sizes consistent.  The parts then run on parts[0]'s stream, and in
+// one form: the flat kernels only when every part does, as on the whole grid.
+struct PartState {
+  cudaStream_t stream;
+  int flat;
+};
+static int group_enter(cgd_handle *const *parts, int32_t n, std::vector<PartState> &saved)
 {
   if (!parts || n < 1) return CGD_ERR_INVALID_ARG;
   for (int r = 0; r < n; ++r) {
@@ -1467,22 +1505,28 @@ static int group_enter(cgd_handle *const *parts, int32_t n, std::vector<cudaStre
   for (int r = 0; r < n; ++r)
     if (int rc = enter(parts[r])) return rc;
   saved.resize(n);
+  int flat = 1;
+  for (int r = 0; r < n; ++r) flat = flat && parts[r]->gp.flat;
   for (int r = 0; r < n; ++r) {
-    saved[r] = parts[r]->stream;
+    saved[r] = PartState{parts[r]->stream, parts[r]->gp.flat};
     parts[r]->stream = parts[0]->stream;
+    parts[r]->gp.flat = flat;
   }
   // work queued on a part's own stream before the call comes first
   for (int r = 1; r < n; ++r) {
     cgd_handle *h = parts[r];
-    cudaEventRecord(h->order_ev, saved[r]);
+    cudaEventRecord(h->order_ev, saved[r].stream);
     cudaStreamWaitEvent(parts[0]->stream, h->order_ev, 0);
   }
   return CGD_OK;
 }
 
-static int group_leave(cgd_handle *const *parts, int32_t n, const std::vector<cudaStream_t> &saved, int rc)
+static int group_leave(cgd_handle *const *parts, int32_t n, const std::vector<PartState> &saved, int rc)
 {
-  for (int r = 0; r < n && r < (int)saved.size(); ++r) parts[r]->stream = saved[r];
+  for (int r = 0; r < n && r < (int)saved.size(); ++r) {
+    parts[r]->stream = saved[r].stream;
+    parts[r]->gp.flat = saved[r].flat;
+  }
   if (rc) return rc;
   return finish(parts[0]);
 }
@@ -1492,7 +1536,7 @@ int cgd_group_rhs(cgd_handle *const *parts, int32_t n, const double *const *U, d
   if (!U || !F) return CGD_ERR_INVALID_ARG;
   for (int r = 0; r < n; ++r)
     if (!U[r] || !F[r] || !is_device_ptr(U[r]) || !is_device_ptr(F[r])) return CGD_ERR_INVALID_ARG;
-  std::vector<cudaStream_t> saved;
+  std::vector<PartState> saved;
   if (int rc = group_enter(parts, n, saved)) return rc;
   std::vector<double *> Ud(n);
   for (int r = 0; r < n; ++r) Ud[r] = const_cast<double *>(U[r]);
@@ -1505,7 +1549,7 @@ int cgd_group_ros_step(cgd_handle *const *parts, int32_t n, double *const *U, do
   if (!U || !(dt > 0) || nsteps < 0) return CGD_ERR_INVALID_ARG;
   for (int r = 0; r < n; ++r)
     if (!U[r] || !is_device_ptr(U[r])) return CGD_ERR_INVALID_ARG;
-  std::vector<cudaStream_t> saved;
+  std::vector<PartState> saved;
   if (int rc = group_enter(parts, n, saved)) return rc;
   int rc = CGD_OK;
   for (int s = 0; s < nsteps && !rc; ++s) rc = part_pieces(parts, n, U, dt, false, nullptr);

@@ -95,8 +95,9 @@ void cgd_destroy(cgd_handle *h);
  * ranks exchange element-node contributions and every rank sums all
  * contributors of a DOF in ascending global (element, node) order, so every
  * rank's DSS'd values, and the column solves that follow, equal the
- * single-process ones bit for bit.  Element-node indices are IF*DoF + ID of
- * the local numbering, 0-based. */
+ * single-process ones bit for bit (in the fast build of parts that run the
+ * same kernels as the whole grid: cgd_set_layers, cgd_flat_form).  Element-node
+ * indices are IF*DoF + ID of the local numbering, 0-based. */
 typedef struct cgd_halo {
   int32_t nnb;                 /* neighbour ranks */
   int32_t nb_boundary;         /* the first nb_boundary local elements touch another rank */
@@ -123,11 +124,25 @@ int cgd_create_part(const cgd_config *cfg, const int64_t *glob, const double *DS
 /* The layer-thickness ratios z(l) / z(0) (nz values, host memory) that the
  * fast build's flat-grid kernels use.  By default a handle takes them from its
  * first element: the sum of J's first node over the element's nodes at level l
- * over that at level 0.  A rank of a decomposed grid is given those of the whole
- * grid's first element, so that its contributions are the single-process ones
- * bit for bit.  z > 0; the factors are formed and checked again.  No effect in
- * the exact build.  No counterpart in the reference. */
+ * over that at level 0.  A part of a decomposed grid (cgd_create_part) is given
+ * those of the whole grid's first element, so that its contributions are the
+ * single-process ones bit for bit; until then it runs the general kernels, whose
+ * results do not depend on the partition either but differ from a flat whole
+ * grid's by rounding.  z > 0; the factors are formed and checked again.  No
+ * effect in the exact build.  No counterpart in the reference. */
 int cgd_set_layers(cgd_handle *h, const double *z);
+
+/* The form of a handle's kernels: *flat = 1 when it runs the flat-grid ones
+ * (fast build, every element's metric a product of horizontal factors and the
+ * layers to 2e-15), else 0.  A grid with one element that is not of that form
+ * runs the general kernels everywhere.  The parts of a decomposed grid judge
+ * their own elements only: cgd_group_* run the flat kernels when all their parts
+ * do; ranks in processes of their own agree once, before their first step -
+ * cgd_flat_form on each, and where any rank has 0, cgd_set_flat_form(h, 0) on
+ * all (Dycore.set_transport does so).  on = 0 refuses the flat kernels, on != 0
+ * lets the check decide again. */
+int cgd_flat_form(cgd_handle *h, int32_t *flat);
+int cgd_set_flat_form(cgd_handle *h, int32_t on);
 
 /* The exchange of one DSS point, supplied by the caller (e.g. NCCL peer
  * sends/receives between processes): nf contribution fields of nz levels per

@@ -55,6 +55,37 @@ def test_two_gloo_ranks(tmp_path):
     assert np.abs(a - 300.0).max() <= 0.01 * 1.0001 and np.abs(b - 300.0).max() <= 0.01 * 1.0001
 
 
+def _flat_worker(rank, world, port, out):
+    import datetime
+
+    import torch.distributed as dist
+    from cgd_b200.parallel import TorchTransport
+    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port))
+    dist.init_process_group("gloo", rank=rank, world_size=world, timeout=datetime.timedelta(seconds=60))
+    try:
+        t = TorchTransport(None)
+        got = [t.all_flat(True), t.all_flat(rank == 0), t.all_flat(False)]
+        with open(os.path.join(out, f"flat{rank}.txt"), "w") as f:
+            f.write(repr(got))
+    finally:
+        dist.destroy_process_group()
+
+
+def test_ranks_agree_on_the_flat_form(tmp_path):
+    """One rank with an element off the flat form sends every rank to the
+    general kernels."""
+    import socket
+
+    import torch.multiprocessing as mp
+    s = socket.socket()
+    s.bind(("127.0.0.1", 0))
+    port = s.getsockname()[1]
+    s.close()
+    mp.start_processes(_flat_worker, args=(2, port, str(tmp_path)), nprocs=2, join=True, start_method="spawn")
+    for r in range(2):
+        assert open(tmp_path / f"flat{r}.txt").read() == repr([True, False, False])
+
+
 def test_reference_arm_runs_on_rank_zero_only(capsys):
     import bench
     from cgd_b200 import physics as Ph
