@@ -381,7 +381,7 @@ int launch_cells_n(cgd_handle *h, const CellArgs &a, int OP, double *cell)
   static std::atomic<unsigned long long> attr{0};
   if (first_on_device(attr))
     CK(cudaFuncSetAttribute(k_cells<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::smem(CELL_MAX)));
-  const dim3 grid((h->nz + CF::LT - 1) / CF::LT, h->NF);
+  const unsigned grid = (unsigned)((h->nz + CF::LT - 1) / CF::LT) * (unsigned)h->NF;
   k_cells<N><<<grid, 256, CF::smem(a.n), h->stream>>>(h->gp, a, h->ointer, OP, cell);
   return CGD_OK;
 }

@@ -63,7 +63,8 @@ __device__ __forceinline__ double exact_quotient(double n, double d, double r)
   return n == 0.0 ? q : n / d;
 }
 
-// One CTA per (element, tile of LT levels).  The nodal values of every
+// One CTA per (element, tile of LT levels), numbered in one dimension: more than
+// 65535 elements are taken.  The nodal values of every
 // quantity are formed once, by one thread per (node, level), level fastest
 // (runs of consecutive levels of a column), into shared planes; then the
 // threads, each holding one sub-cell's N^2 weights in registers, walk the
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(256, N == 5 ? 3 : 4) k_cells(const GP P, const
   extern __shared__ __align__(16) double sc[];
   double *srho = sc + (size_t)A.n * PL, *srr = srho + PL, *tx = srr + PL, *ty = tx + PL;
   const int nz = P.nz, OP2 = OP * OP;
-  const int IF = blockIdx.y, l0 = blockIdx.x * LT;
+  const int tiles = (nz + LT - 1) / LT, IF = blockIdx.x / tiles, l0 = (blockIdx.x % tiles) * LT;
   const int t = threadIdx.x;
   const int lvl = t % LT, ID = t / LT, l = l0 + lvl;
   const bool act = ID < DoF && l < nz;

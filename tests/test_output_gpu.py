@@ -147,3 +147,48 @@ def test_vtk_output_file(built_lib, cuda_ok, case, tmp_path):
     data2 = output.read_vtu(p2)[4]
     assert all(np.array_equal(data2[n], data[n]) for n in data)
     d.close()
+
+
+def test_more_than_65535_elements(built_lib, cuda_ok):
+    """66150 elements (nPanel 105, p 1): the interpolation of a column, of a
+    ratio, of w and of the state's quantities against the same sums in numpy."""
+    import torch
+    from cgd_b200 import Dycore, _lib, output
+    from cgd_b200 import grid as G
+    n, nz, OP = 105, 2, 2
+    g = G.init_grid_sphere_device(n, 1, G.vertical_uniform(nz, 1000.0), 1000.0, 6.371e6)
+    d = Dycore(g, 0, (0.0, 0.0, 0.0))
+    assert d.NF > 65535
+    rng = np.random.Generator(np.random.PCG64(5))
+    U = np.asfortranarray(rng.uniform(0.5, 1.5, d.shape))
+    U[..., 4] *= 300.0
+    inter = output.vtk_inter(1, OP, g.xw)
+    glob = np.asarray(g.glob) - 1                                       # (DoF, NF)
+
+    def cells(node):                                                    # node(iD): (nz, NF)
+        out = np.zeros((OP, OP, nz, d.NF))
+        for iD in range(4):
+            out = out + inter[:, :, iD % 2, iD // 2][:, :, None, None] * node(iD)[None, None]
+        return out
+
+    f = lambda k: np.asfortranarray(U[..., k])
+    col = lambda a: lambda iD: a[:, glob[iD]]
+    assert np.array_equal(d.interpolate(f(1), inter), cells(col(f(1))))
+    ref = np.zeros((OP, OP, nz, d.NF))
+    for iD in range(4):
+        w = inter[:, :, iD % 2, iD // 2][:, :, None, None]
+        ref = ref + w * col(f(2))(iD)[None, None] / col(f(0))(iD)[None, None]
+    assert np.array_equal(d.interpolate(f(2), inter, rhoc=f(0)), ref)
+    dX = g.dXdxI.cpu().numpy() if hasattr(g.dXdxI, "cpu") else np.asarray(g.dXdxI).T   # (NF, nz, DoF, 2, 3, 3)
+
+    def wbar(iD):
+        u, v, w = (col(f(k))(iD) for k in (1, 2, 3))
+        m = dX[:, 0, iD, 0]                                             # [.., b, a] = dXdxI(a, b)
+        below = np.vstack([-(u[0] * m[:, 0, 2] + v[0] * m[:, 1, 2]) / m[:, 2, 2], w[:-1]])
+        return 0.5 * (w + below)
+
+    assert np.array_equal(d.interpolate_wb(f(1), f(2), f(3), inter), cells(wbar))
+    out = d.output_fields(U, [_lib.OUT_RHO, _lib.OUT_WB_UV], inter).reshape(2, d.NF, nz, OP, OP)
+    for o, r in zip(out, (cells(col(f(0))), cells(wbar))):
+        assert np.array_equal(o, r.transpose(3, 2, 1, 0))
+    d.close()
