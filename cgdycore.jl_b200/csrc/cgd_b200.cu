@@ -374,27 +374,101 @@ void column(cgd_handle *h, const ColArgs &a)
   else column_t<MODE, false>(h, a);
 }
 
-template <int N>
-int launch_cells_n(cgd_handle *h, const CellArgs &a, int OP, double *cell)
+// The output launches of n quantities, with up to 25 of a quantity's sub-cells a
+// thread.  A launch of few CTAs is bound by a thread's chain of sums and by the
+// second launch itself: below CELLS_SMALL CTAs a thread takes 4 (9 of an odd
+// OrdPrint) and k_cells starts while k_cells_nodal ends.  Above, its waiting CTAs
+// would keep that kernel's out: nPanel 60, p 1, nz 40, vorticity 97 -> 107 us.
+constexpr unsigned CELLS_SMALL = 2 * 148;
+
+template <int N, int CH>
+void launch_cells_c(cgd_handle *h, const CellArgs &a, int n, int OP, double *cell, bool overlap)
 {
-  using CF = CellCfg<N>;
-  static std::atomic<unsigned long long> attr{0};
-  if (first_on_device(attr))
-    CK(cudaFuncSetAttribute(k_cells<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::smem(CELL_MAX)));
-  const unsigned grid = (unsigned)((h->nz + CF::LT - 1) / CF::LT) * (unsigned)h->NF;
-  k_cells<N><<<grid, 256, CF::smem(a.n), h->stream>>>(h->gp, a, h->ointer, OP, cell);
-  return CGD_OK;
+  const long long total = (long long)h->nz * h->NF;
+  const unsigned groups = (OP * OP + CH - 1) / CH;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((total + CELL_THREADS - 1) / CELL_THREADS) * groups, n);
+  cfg.blockDim = dim3(CELL_THREADS);
+  cfg.stream = h->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_cells<N, CH>, (const GP)h->gp, (const CellArgs)a, (const double *)h->ointer, OP * OP, cell);
 }
 
-int launch_cells(cgd_handle *h, const CellArgs &a, int OP, double *cell)
+template <int N>
+void launch_cells_n(cgd_handle *h, NodalArgs na, const CellArgs &a, int n, int OP, double *cell)
 {
-  switch (h->N) {
-    case 2: return launch_cells_n<2>(h, a, OP, cell);
-    case 3: return launch_cells_n<3>(h, a, OP, cell);
-    case 4: return launch_cells_n<4>(h, a, OP, cell);
-    default: return launch_cells_n<5>(h, a, OP, cell);
+  using CF = NodalCfg<N>;
+  const size_t S = (size_t)h->nz * h->NumG;
+  na.colblocks = na.p || na.th ? (unsigned)((S + CF::THREADS - 1) / CF::THREADS) : 0;
+  na.w0blocks = na.w0[0] || na.w0[1] ? (unsigned)((h->NF * CF::DoF + CF::THREADS - 1) / CF::THREADS) : 0;
+  const unsigned tiles = na.rot ? (unsigned)((h->nz + CF::LT - 1) / CF::LT) * (unsigned)h->NF : 0;
+  const unsigned nodal = na.colblocks + na.w0blocks + tiles;
+  const bool small = (unsigned)(((long long)h->nz * h->NF + CELL_THREADS - 1) / CELL_THREADS) * n < CELLS_SMALL;
+  const bool overlap = small && nodal;
+  na.overlap = overlap;
+  if (nodal > tiles) k_cells_nodal<N, true><<<nodal, CF::THREADS, 0, h->stream>>>(h->gp, na);
+  else if (nodal) k_cells_nodal<N, false><<<nodal, CF::THREADS, 0, h->stream>>>(h->gp, na);
+  const int CH = OP == 1 ? 1 : small ? (OP % 2 ? 9 : 4) : OP == 6 ? 18 : OP == 8 ? 16 : std::min(OP * OP, 25);
+  switch (CH) {
+    case 1: launch_cells_c<N, 1>(h, a, n, OP, cell, overlap); break;
+    case 4: launch_cells_c<N, 4>(h, a, n, OP, cell, overlap); break;
+    case 9: launch_cells_c<N, 9>(h, a, n, OP, cell, overlap); break;
+    case 16: launch_cells_c<N, 16>(h, a, n, OP, cell, overlap); break;
+    case 18: launch_cells_c<N, 18>(h, a, n, OP, cell, overlap); break;
+    default: launch_cells_c<N, 25>(h, a, n, OP, cell, overlap); break;   // OrdPrint 7: 25 + 24
   }
 }
+
+// The quantities of an output call, the next up to CELL_MAX of them a launch of
+// k_cells; what is no column of the state is formed first, once a call, in the
+// handle's phase-1 contributions (no call reads those of an earlier one).
+struct CellList {
+  cgd_handle *h;
+  int OP;
+  double *cell;
+  NodalArgs na{};
+  CellArgs a{};
+  int n = 0;
+
+  CellList(cgd_handle *h_, int OP_, double *cell_, const double *U) : h(h_), OP(OP_), cell(cell_)
+  {
+    const size_t fs = (size_t)h->nz * h->NumG;
+    if (U) {
+      a.rho = na.rho = U;
+      na.u = U + fs;
+      na.v = U + 2 * fs;
+      na.rhoth = U + 4 * fs;
+    }
+  }
+  // rot, p, th, w0 (2): of the size of an element-node array each, or less
+  double *work(size_t k) const { return h->C1 + k * h->DoF * h->nz * h->NF; }
+  const double *vort() { return na.rot = work(0); }
+  const double *pres() { return na.p = work(1); }
+  const double *pott() { return na.th = work(2); }
+  const double *surface(bool uv) { return na.w0[uv] = work(3 + uv); }
+  void add(int op, const double *c, const double *w0 = nullptr)
+  {
+    if (n == CELL_MAX) flush();
+    a.f[n++] = CellOp{op, c, w0};
+  }
+  void flush()
+  {
+    if (!n) return;
+    switch (h->N) {
+      case 2: launch_cells_n<2>(h, na, a, n, OP, cell); break;
+      case 3: launch_cells_n<3>(h, na, a, n, OP, cell); break;
+      case 4: launch_cells_n<4>(h, na, a, n, OP, cell); break;
+      default: launch_cells_n<5>(h, na, a, n, OP, cell); break;
+    }
+    cell += (size_t)n * OP * OP * h->nz * h->NF;
+    n = 0;
+    na.p = na.th = na.rot = na.w0[0] = na.w0[1] = nullptr;
+  }
+};
 
 // Event between two kernels of a step launched without the graph (the
 // profiled step, see cgd_ros_step).
@@ -1683,11 +1757,10 @@ int cgd_interpolate(cgd_handle *h, const double *c, const double *rhoc, const do
   if (int rc = out_input(h, rhoc, 1, &rd)) return rc;
   const size_t n = out_count(h, OrdPrint);
   if (int rc = out_cells(h, cCell, n, &od)) return rc;
-  CellArgs a{};
-  a.n = 1;
-  a.f[0] = CellOp{rd ? CELL_C_RHO : CELL_C, cd, nullptr, nullptr};
-  a.rho = rd;
-  if (int rc = launch_cells(h, a, OrdPrint, od)) return rc;
+  CellList q(h, OrdPrint, od, nullptr);
+  q.a.rho = rd;
+  q.add(rd ? CELL_C_RHO : CELL_C, cd);
+  q.flush();
   if (od != cCell) CK(cudaMemcpyAsync(cCell, od, n * 8, cudaMemcpyDeviceToHost, h->stream));
   return finish(h);
 }
@@ -1705,10 +1778,11 @@ int cgd_interpolate_wb(cgd_handle *h, const double *u, const double *v, const do
   if (int rc = out_input(h, w, 2, &wd)) return rc;
   const size_t n = out_count(h, OrdPrint);
   if (int rc = out_cells(h, cCell, n, &od)) return rc;
-  CellArgs a{};
-  a.n = 1;
-  a.f[0] = CellOp{CELL_WB, wd, ud, vd};
-  if (int rc = launch_cells(h, a, OrdPrint, od)) return rc;
+  CellList q(h, OrdPrint, od, nullptr);
+  q.na.u = ud;
+  q.na.v = vd;
+  q.add(CELL_WB, wd, q.surface(true));
+  q.flush();
   if (od != cCell) CK(cudaMemcpyAsync(cCell, od, n * 8, cudaMemcpyDeviceToHost, h->stream));
   return finish(h);
 }
@@ -1722,11 +1796,9 @@ int cgd_interpolate_vort(cgd_handle *h, const double *U, const double *inter, in
   if (int rc = stage_in(h, U, h->Ubuf, true, &Ud)) return rc;
   const size_t n = out_count(h, OrdPrint);
   if (int rc = out_cells(h, cCell, n, &od)) return rc;
-  const size_t fs = (size_t)h->nz * h->NumG;
-  CellArgs a{};
-  a.n = 1;
-  a.f[0] = CellOp{CELL_VORT, nullptr, Ud + fs, Ud + 2 * fs};
-  if (int rc = launch_cells(h, a, OrdPrint, od)) return rc;
+  CellList q(h, OrdPrint, od, Ud);
+  q.add(CELL_NODE, q.vort());
+  q.flush();
   if (od != cCell) CK(cudaMemcpyAsync(cCell, od, n * 8, cudaMemcpyDeviceToHost, h->stream));
   return finish(h);
 }
@@ -1747,36 +1819,22 @@ int cgd_output_fields(cgd_handle *h, const double *U, const int32_t *fields, int
   const size_t n = out_count(h, OrdPrint);
   if (int rc = out_cells(h, out, n * nfields, &od)) return rc;
   const size_t fs = (size_t)h->nz * h->NumG;
-  const double *rho = Ud, *u = Ud + fs, *v = Ud + 2 * fs, *w = Ud + 3 * fs, *rth = Ud + 4 * fs;
-  // up to CELL_MAX quantities, at most one of them the vorticity, per launch
-  for (int k0 = 0; k0 < nfields;) {
-    CellArgs a{};
-    a.rho = rho;
-    a.rhoth = rth;
-    bool vort = false;
-    int k = k0;
-    for (; k < nfields && a.n < CELL_MAX; ++k) {
-      CellOp &f = a.f[a.n];
-      switch (fields[k]) {
-        case CGD_OUT_RHO: f = CellOp{CELL_C, rho, nullptr, nullptr}; break;
-        case CGD_OUT_U: f = CellOp{CELL_C, u, nullptr, nullptr}; break;
-        case CGD_OUT_V: f = CellOp{CELL_C, v, nullptr, nullptr}; break;
-        case CGD_OUT_WB: f = CellOp{CELL_WB, w, u, u}; break;
-        case CGD_OUT_WB_UV: f = CellOp{CELL_WB, w, u, v}; break;
-        case CGD_OUT_TH: f = CellOp{CELL_POTT, nullptr, nullptr, nullptr}; break;
-        case CGD_OUT_PRES: f = CellOp{CELL_PRES, nullptr, nullptr, nullptr}; break;
-        case CGD_OUT_VORT: f = CellOp{CELL_VORT, nullptr, u, v}; break;
-        default:   // tracer ratio rho*q / rho
-          f = CellOp{CELL_C_RHO, Ud + (size_t)(5 + fields[k] - CGD_OUT_TR) * fs, nullptr, nullptr};
-          break;
-      }
-      if (f.op == CELL_VORT && vort) break;   // the next launch's
-      vort = vort || f.op == CELL_VORT;
-      ++a.n;
+  const double *rho = Ud, *u = Ud + fs, *v = Ud + 2 * fs, *w = Ud + 3 * fs;
+  CellList q(h, OrdPrint, od, Ud);
+  for (int k = 0; k < nfields; ++k) {
+    switch (fields[k]) {
+      case CGD_OUT_RHO: q.add(CELL_C, rho); break;
+      case CGD_OUT_U: q.add(CELL_C, u); break;
+      case CGD_OUT_V: q.add(CELL_C, v); break;
+      case CGD_OUT_WB: q.add(CELL_WB, w, q.surface(false)); break;
+      case CGD_OUT_WB_UV: q.add(CELL_WB, w, q.surface(true)); break;
+      case CGD_OUT_TH: q.add(CELL_C, q.pott()); break;
+      case CGD_OUT_PRES: q.add(CELL_C, q.pres()); break;
+      case CGD_OUT_VORT: q.add(CELL_NODE, q.vort()); break;
+      default: q.add(CELL_C_RHO, Ud + (size_t)(5 + fields[k] - CGD_OUT_TR) * fs); break;   // tracer ratio rho*q / rho
     }
-    if (int rc = launch_cells(h, a, OrdPrint, od + (size_t)k0 * n)) return rc;
-    k0 = k;
   }
+  q.flush();
   if (od != out) CK(cudaMemcpyAsync(out, od, n * nfields * 8, cudaMemcpyDeviceToHost, h->stream));
   return finish(h);
 }

@@ -1,8 +1,8 @@
-// cgd_output.cuh - interpolation of the state to the output sub-cells.
+// cgd_output.cuh - interpolation of the state to sub-cells for the output files.
 //
-// The reference writes its VTK output from OrdPrint x OrdPrint sub-cells per
-// element and layer: each cell value is the element's GLL interpolant at the
-// cell centre, Inter[I,J,iP,jP] = L_iP(xi_I) L_jP(eta_J)
+// Each element and layer is divided into OrdPrint x OrdPrint sub-cells; the
+// cell value of a quantity c is the interpolating polynomial at the sub-cell
+// centre, Inter[I,J,iP,jP] = L_iP(xi_I) L_jP(eta_J)
 // (src/Outputs/vtkSphere.jl:199-219), applied to the nodal values gathered
 // through Glob (InterpolateKernel!, src/Outputs/vtkOutputKernel.jl:49-74).
 // k_cells evaluates the same sums in the same order, several quantities at once:
@@ -18,6 +18,28 @@
 // sum_I D(i,I) tx(I,j) followed by sum_J D(j,J) ty(i,J), from 0.
 // Inter is Fortran-ordered (OrdPrint, OrdPrint, N, N); cCell is
 // (OrdPrint, OrdPrint, nz, NF).
+//
+// Two launches.  k_cells_nodal forms what is not a column of the state: the
+// pressure and the potential temperature once per column and level, the
+// vorticity once per element node and level, the surface w once per element
+// node (only those asked for; no launch for none).  k_cells then is a thread per
+// (element, level) and quantity, which gathers the N^2 nodal values (neighbouring
+// threads: neighbouring levels of one column) and keeps up to 25 sub-cells' sums
+// in registers.  One kernel with the nodal values of every quantity in shared
+// planes, as before, spent its time in the chain index - columns - pow - barrier -
+// curl - barrier - sums of 10 levels a CTA; with one sub-cell, or one quantity,
+// most of its threads idled.  Calls on nPanel 30, p 4, nz 45, two tracers, us:
+//
+//                      OrdPrint 1        OrdPrint 4        OrdPrint 8
+//   nine quantities    966 -> 312        941 -> 475        1841 -> 1223
+//   rho alone          204 -> 39         218 -> 52
+//   a tracer alone     656 -> 55         351 -> 95
+//   vorticity alone    311 -> 145        327 -> 161
+//
+// and nPanel 60, nz 64, seven quantities, OrdPrint 1 2718 -> 1260; nPanel 6, nz 10
+// 37 -> 36 (of these some 25 us are the call's own).  k_cells_nodal reads 0.26 GB
+// of metric at 4.0 TB/s (nPanel 20: 87 us under a profiler), k_cells moves 3.1
+// TB/s (50 us) and waits for its gathers.
 #pragma once
 #include "cgd_kernels.cuh"
 
@@ -33,163 +55,221 @@ __device__ __forceinline__ double pott_dry(const GP &P, double rho, double p)
   return pow(P.p0 / p, P.kappa) * T;   // (p0/p)^(Rd/Cpd) * T
 }
 
-// What a cell value interpolates.
-enum { CELL_C = 0, CELL_C_RHO, CELL_PRES, CELL_POTT, CELL_WB, CELL_VORT };
+// Levels of a vorticity tile; threads (node, level), level fastest.
+template <int N>
+struct NodalCfg {
+  static constexpr int DoF = N * N, LT = N == 2 ? 32 : 16, RS = DoF | 1, THREADS = LT * DoF;
+};
+
+// What k_cells_nodal forms (null: not wanted): columns p and th of rho and
+// rhoth; the surface w, -(a d31 + b d32) / d33 of the lowest lower node (no
+// normal flow), [IF][ID], for (a, b) = (u, u) in w0[0] and (u, v) in w0[1]; the
+// vorticity rot ([IF][ID][nz]) of u and v.  The first colblocks CTAs take the
+// columns (bound by exp, log and pow), the next w0blocks the surface, the others
+// a tile of an element each (bound by its ten metric values a node and level).
+struct NodalArgs {
+  const double *rho, *rhoth, *u, *v;
+  double *p, *th, *w0[2], *rot;
+  unsigned colblocks, w0blocks;
+  bool overlap;   // k_cells may start now
+};
+
+template <int N, bool COLS>   // COLS: more than the vorticity
+__global__ void __launch_bounds__(NodalCfg<N>::THREADS) k_cells_nodal(const GP P, const NodalArgs A)
+{
+  using CF = NodalCfg<N>;
+  constexpr int DoF = CF::DoF, LT = CF::LT, RS = CF::RS;
+  const int nz = P.nz, t = threadIdx.x;
+  if (A.overlap) asm volatile("griddepcontrol.launch_dependents;\n");   // k_cells waits for this grid's end itself
+  if (COLS && blockIdx.x < A.colblocks) {
+    const size_t i = (size_t)blockIdx.x * CF::THREADS + t;
+    if (i >= (size_t)nz * P.NumG) return;
+    const double p = pressure_dry(P, A.rhoth[i]);
+    if (A.p) A.p[i] = p;
+    if (A.th) A.th[i] = pott_dry(P, A.rho[i], p);
+    return;
+  }
+  if (COLS && blockIdx.x < A.colblocks + A.w0blocks) {
+    const int n = (blockIdx.x - A.colblocks) * CF::THREADS + t;
+    if (n >= P.NF * DoF) return;
+    const size_t o = (size_t)nz * P.glob[n], cs = (size_t)DoF * nz;
+    const double *m = P.met + ((size_t)(n / DoF) * NCOMP * DoF + n % DoF) * nz;
+    const double u = A.u[o], d31 = m[C_D31_0 * cs], d32 = m[C_D32_0 * cs], d33 = m[C_D33_0 * cs];
+    if (A.w0[0]) A.w0[0][n] = -(u * d31 + u * d32) / d33;
+    if (A.w0[1]) A.w0[1][n] = -(u * d31 + A.v[o] * d32) / d33;
+    return;
+  }
+  __shared__ double tx[LT * RS], ty[LT * RS];
+  const unsigned b = COLS ? blockIdx.x - A.colblocks - A.w0blocks : blockIdx.x, tiles = (nz + LT - 1) / LT;
+  const int IF = b / tiles, lvl = t % LT, ID = t / LT, l = (b % tiles) * LT + lvl;
+  const bool act = l < nz;
+  const int i = ID % N, j = ID / N, row = lvl * RS;
+  double J = 1.0;
+  if (act) {
+    const size_t cs = (size_t)DoF * nz, o = l + (size_t)nz * P.glob[(size_t)IF * DoF + ID];
+    const double *mt = P.met + ((size_t)IF * NCOMP * DoF + ID) * nz + l;
+    const double u = A.u[o], v = A.v[o];
+    tx[row + ID] = (mt[C_D11_0 * cs] + mt[C_D11_1 * cs]) * v - (mt[C_D12_0 * cs] + mt[C_D12_1 * cs]) * u;
+    ty[row + ID] = (mt[C_D21_0 * cs] + mt[C_D21_1 * cs]) * v - (mt[C_D22_0 * cs] + mt[C_D22_1 * cs]) * u;
+    J = mt[C_J0 * cs] + mt[C_J1 * cs];
+  }
+  __syncthreads();
+  if (!act) return;
+  double acc = 0.0;
+#pragma unroll
+  for (int I = 0; I < N; ++I) acc += P.D[i + N * I] * tx[row + I + N * j];
+#pragma unroll
+  for (int k = 0; k < N; ++k) acc += P.D[j + N * k] * ty[row + i + N * k];
+  A.rot[((size_t)IF * DoF + ID) * nz + l] = acc / J;
+}
+
+// What a cell value interpolates: a column c, c over rho, the layer mean of the
+// column c = w with w0 at the surface, or the element-node array c.
+enum { CELL_C = 0, CELL_C_RHO, CELL_WB, CELL_NODE };
 
 // One launch's quantities: cell array k (n values each, back to back) is kind
-// op[k].op of the columns c (and, for CELL_WB, u, v; for CELL_VORT, u and v).
+// op of f[k].
 constexpr int CELL_MAX = 16;
 struct CellOp {
   int op;
-  const double *c, *u, *v;
+  const double *c, *w0;
 };
 struct CellArgs {
   CellOp f[CELL_MAX];
-  int n;
-  const double *rho, *rhoth;   // (nz, NumG); what CELL_C_RHO divides by, what the pressure is of
+  const double *rho;   // (nz, NumG), what CELL_C_RHO divides by
 };
 
 // n / d with r = 1 / d: the correctly rounded quotient by two Newton
-// corrections of n r, whose residuals are exact; outside the range where they
-// are, the division itself.
+// corrections of n r, whose residuals are exact (Markstein's theorem: from an
+// approximation within one unit in the last place, with r correctly rounded,
+// the second is correctly rounded).  For n zero or in 2^-400 .. 2^500 and d in
+// 2^-400 .. 2^400, where nothing overflows or loses bits to underflow.
 __device__ __forceinline__ double exact_quotient(double n, double d, double r)
 {
   double q = n * r;
-  const double a = fabs(q);
-  if (a > 1e-280 && a < 1e280) {
-    q = __fma_rn(__fma_rn(-q, d, n), r, q);
-    return __fma_rn(__fma_rn(-q, d, n), r, q);
-  }
-  return n == 0.0 ? q : n / d;
+  q = __fma_rn(__fma_rn(-q, d, n), r, q);
+  return __fma_rn(__fma_rn(-q, d, n), r, q);
 }
 
-// One CTA per (element, tile of LT levels), numbered in one dimension: more than
-// 65535 elements are taken.  The nodal values of every
-// quantity are formed once, by one thread per (node, level), level fastest
-// (runs of consecutive levels of a column), into shared planes; then the
-// threads, each holding one sub-cell's N^2 weights in registers, walk the
-// (quantity, level) pairs and write runs of consecutive cells.  One kernel
-// per quantity and one thread per cell, as before, gathered the columns again
-// for every sub-cell, evaluated the pressure's exp and log N^2 times for each,
-// and wrote OrdPrint^2 values apart: nPanel 30, nz 45, nine quantities on
-// 4 x 4 sub-cells 4.80 ms.
-template <int N>
-struct CellCfg {
-  static constexpr int DoF = N * N, LT = 256 / DoF;
-  static constexpr int RS = (DoF + 2) & ~1;   // row of a plane: even, so that two nodes are one 16-byte load
-  static constexpr int PL = LT * RS;
-  static size_t smem(int nq) { return ((size_t)(nq + 4) * PL) * sizeof(double); }   // planes, rho, 1/rho, tx, ty
-};
-
-template <int N>
-__global__ void __launch_bounds__(256, N == 5 ? 3 : 4) k_cells(const GP P, const CellArgs A, const double *__restrict__ inter, int OP,
-                                               double *__restrict__ cell)
+// |x| in 2^lo .. 2^hi (below 2^(hi+1)), zero too where it may be.
+__device__ __forceinline__ bool in_range(double x, int lo, int hi, bool zero)
 {
-  using CF = CellCfg<N>;
-  constexpr int DoF = CF::DoF, LT = CF::LT, RS = CF::RS, PL = CF::PL;
-  extern __shared__ __align__(16) double sc[];
-  double *srho = sc + (size_t)A.n * PL, *srr = srho + PL, *tx = srr + PL, *ty = tx + PL;
-  const int nz = P.nz, OP2 = OP * OP;
-  const int tiles = (nz + LT - 1) / LT, IF = blockIdx.x / tiles, l0 = (blockIdx.x % tiles) * LT;
-  const int t = threadIdx.x;
-  const int lvl = t % LT, ID = t / LT, l = l0 + lvl;
-  const bool act = ID < DoF && l < nz;
-  const size_t cs = (size_t)DoF * nz;
-  const int si = lvl * RS + ID;
-  const double *mt = P.met + ((size_t)IF * NCOMP * DoF + ID) * nz + l;
-  size_t o = 0;
-  double rho = 1.0, p = 0.0, pt = 0.0;
-  int vort = -1;
-  if (act) {
-    o = l + (size_t)nz * P.glob[(size_t)IF * DoF + ID];
-    bool need_rho = false, need_p = false, div_rho = false, need_pt = false;
-    for (int k = 0; k < A.n; ++k) {
-      need_rho = need_rho || A.f[k].op == CELL_C_RHO || A.f[k].op == CELL_POTT;
-      need_p = need_p || A.f[k].op == CELL_PRES || A.f[k].op == CELL_POTT;
-      div_rho = div_rho || A.f[k].op == CELL_C_RHO;
-      need_pt = need_pt || A.f[k].op == CELL_POTT;
+  const int e = ((__double2hiint(x) >> 20) & 0x7ff) - 1023;
+  return (e >= lo && e <= hi) || (zero && x == 0.0);
+}
+
+constexpr int CELL_THREADS = 128;
+
+// CH sub-cells a thread; blockIdx.y: quantity; blockIdx.x: group of CH sub-cells
+// (fastest, so that the groups' halves of a cache line come together), pairs.
+// CH > 1: the weights are read from shared memory, as broadcasts, and the sums go
+// out through it, a warp's in runs of CH values.
+template <int N, int CH>
+__global__ void __launch_bounds__(CELL_THREADS, CH == 1 ? 8 : CH <= 9 ? 6 : CH <= 18 ? 5 : 4) k_cells(const GP P, const CellArgs A, const double *__restrict__ inter,
+                                                        int OP2, double *__restrict__ cell)
+{
+  constexpr int DoF = N * N, CS = CH | 1;
+  __shared__ __align__(16) double sw[CH > 1 ? DoF * CH : 1];
+  __shared__ double so[CH > 1 ? CELL_THREADS * CS : 1];
+  const int nz = P.nz, t = threadIdx.x, groups = (OP2 + CH - 1) / CH;
+  const int c0 = blockIdx.x % groups * CH, nc = min(CH, OP2 - c0);
+  const long long total = (long long)nz * P.NF, first = (long long)(blockIdx.x / groups) * CELL_THREADS;
+  const bool in = first + t < total;
+  const long long x = in ? first + t : total - 1;
+  const int IF = (int)(x / nz), l = (int)(x - (long long)IF * nz);
+  const int *gl = P.glob + (size_t)IF * DoF;
+  if (CH > 1) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(gl));   // while the weights come
+  bool plain = true;   // every weight zero or in 2^-100 .. 2^99
+  if (CH > 1) {
+    for (int y = t; y < DoF * CH; y += CELL_THREADS) {
+      const int n = y / CH, c = y % CH;
+      const double w = c < nc ? inter[c0 + c + (size_t)OP2 * n] : 0.0;
+      sw[y] = w;
+      plain = plain && in_range(w, -100, 98, true);
     }
-    if (need_rho) rho = A.rho[o];
-    if (div_rho) {
-      srho[si] = rho;
-      srr[si] = 1.0 / rho;
-    }
-    if (need_p) p = pressure_dry(P, A.rhoth[o]);
-    if (need_pt) pt = pott_dry(P, rho, p);
+    plain = __syncthreads_and(plain);
   }
-  // the columns' values first, all of a thread's loads in flight at once
-  double x[CELL_MAX];
+  auto weight = [&](int n, int c) { return CH > 1 ? sw[n * CH + c] : inter[c0 + (size_t)OP2 * n]; };
+  const CellOp f = A.f[blockIdx.y];
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");   // k_cells_nodal's arrays
+  double acc[CH];
 #pragma unroll
-  for (int k = 0; k < CELL_MAX; ++k) {
-    x[k] = 0.0;
-    if (act && k < A.n && A.f[k].c && A.f[k].op != CELL_WB) x[k] = A.f[k].c[o];
-  }
+  for (int c = 0; c < CH; ++c) acc[c] = 0.0;
+  // sum of weight * value(n) over the nodes in ascending order
+  auto sums = [&](auto &&value) {
 #pragma unroll
-  for (int k = 0; k < CELL_MAX; ++k) {
-    if (act && k < A.n) {
-      const int op = A.f[k].op;
-      sc[(size_t)k * PL + si] = op == CELL_PRES ? p : op == CELL_POTT ? pt : x[k];
+    for (int n = 0; n < DoF; ++n) {
+      const double y = value(n);
+#pragma unroll
+      for (int c = 0; c < CH; ++c) acc[c] += weight(n, c) * y;
     }
-  }
-  for (int k = 0; k < A.n; ++k) {
-    const CellOp f = A.f[k];
-    if (f.op == CELL_VORT) {   // uniform: at most one per launch
-      vort = k;
-      if (act) {
-        const double u = f.u[o], v = f.v[o];
-        tx[si] = (mt[C_D11_0 * cs] + mt[C_D11_1 * cs]) * v - (mt[C_D12_0 * cs] + mt[C_D12_1 * cs]) * u;
-        ty[si] = (mt[C_D21_0 * cs] + mt[C_D21_1 * cs]) * v - (mt[C_D22_0 * cs] + mt[C_D22_1 * cs]) * u;
+  };
+  // the same with divisions: a row's loads first (their slow paths keep loads
+  // from being moved ahead of them)
+  auto rows = [&](auto &&load, auto &&add) {
+#pragma unroll 1
+    for (int jn = 0; jn < N; ++jn) {
+      double z[N][2];
+#pragma unroll
+      for (int k = 0; k < N; ++k) load(jn * N + k, z[k]);
+#pragma unroll
+      for (int k = 0; k < N; ++k) add(jn * N + k, z[k]);
+    }
+  };
+  if (f.op == CELL_C) {
+    sums([&](int n) { return f.c[l + (size_t)nz * gl[n]]; });
+  } else if (f.op == CELL_NODE) {
+    const double *e = f.c + (size_t)IF * DoF * nz + l;
+    sums([&](int n) { return e[(size_t)n * nz]; });
+  } else if (f.op == CELL_WB) {
+    // the reference halves the weight, the same value
+    sums([&](int n) {
+      const size_t o = l + (size_t)nz * gl[n];
+      const double *below = l > 0 ? f.c + o - 1 : f.w0 + IF * DoF + n;
+      return 0.5 * (f.c[o] + *below);
+    });
+  } else if (CH == 1) {
+    rows([&](int n, double *z) {
+      const size_t o = l + (size_t)nz * gl[n];
+      z[0] = f.c[o]; z[1] = A.rho[o];
+    }, [&](int n, const double *z) { acc[0] += weight(n, 0) * z[0] / z[1]; });
+  } else {
+    // one division a node instead of one a sub-cell, with the same quotients
+    rows([&](int n, double *z) {
+      const size_t o = l + (size_t)nz * gl[n];
+      z[0] = f.c[o]; z[1] = A.rho[o];
+    }, [&](int n, const double *z) {
+      const double y = z[0], d = z[1];
+      if (plain && in_range(d, -400, 399, false) && in_range(y, -300, 399, true)) {
+        const double r = 1.0 / d;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) acc[c] += exact_quotient(weight(n, c) * y, d, r);
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < nc; ++c) so[t * CS + c] = weight(n, c) * y / d;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) acc[c] += so[t * CS + c];
       }
-    } else if (f.op == CELL_WB && act) {
-      // 0.5 (w(l) + w(l-1)), in the lowest layer 0.5 (w(1) + w0) with w0 =
-      // -(u d31 + v d32) / d33 of the lower node (no normal flow); the
-      // reference halves the weight, the same value
-      const double below = l == 0 ? -(f.u[o] * mt[C_D31_0 * cs] + f.v[o] * mt[C_D32_0 * cs]) / mt[C_D33_0 * cs] : f.c[o - 1];
-      sc[(size_t)k * PL + si] = 0.5 * (f.c[o] + below);
-    }
+    });
   }
-  __syncthreads();
-  if (vort >= 0) {
-    if (act) {
-      const int i = ID % N, j = ID / N, row = lvl * RS;
-      double acc = 0.0;
-#pragma unroll
-      for (int I = 0; I < N; ++I) acc += P.D[i + N * I] * tx[row + I + N * j];
-#pragma unroll
-      for (int J = 0; J < N; ++J) acc += P.D[j + N * J] * ty[row + i + N * J];
-      sc[(size_t)vort * PL + si] = acc / (mt[C_J0 * cs] + mt[C_J1 * cs]);
-    }
-    __syncthreads();
+  double *out = cell + (size_t)blockIdx.y * OP2 * total;
+  if (CH == 1) {
+    if (in) out[x * OP2 + c0] = acc[0];
+    return;
   }
-  // the cells: thread t holds the weights of sub-cell t % OP2
-  const int step = 256 / OP2;          // (quantity, level) pairs in flight
-  const int cI = t % OP2, p0 = t / OP2;
-  if (p0 >= step) return;
-  double w[DoF];
+  const int warp = t & ~31, lane = t & 31;
 #pragma unroll
-  for (int n = 0; n < DoF; ++n) w[n] = inter[cI + (size_t)OP2 * n];
-  const int nl = min(LT, nz - l0);
-  const size_t per = (size_t)OP2 * nz * P.NF;
-  double *out = cell + cI + (size_t)OP2 * (l0 + (size_t)nz * IF);
-  for (int q = p0; q < A.n * nl; q += step) {
-    const int k = q / nl, lz = q - k * nl;
-    const double *s = sc + (size_t)k * PL + lz * RS;
-    double acc = 0.0;
-    if (A.f[k].op == CELL_C_RHO) {
-      const double *sr = srho + lz * RS, *si2 = srr + lz * RS;
-#pragma unroll
-      for (int n = 0; n < DoF; ++n) acc += exact_quotient(w[n] * s[n], sr[n], si2[n]);
-    } else {
-      const double2 *s2 = reinterpret_cast<const double2 *>(s);
-#pragma unroll
-      for (int n = 0; n + 1 < DoF; n += 2) {
-        const double2 x = s2[n / 2];
-        acc += w[n] * x.x;
-        acc += w[n + 1] * x.y;
-      }
-      if (DoF % 2) acc += w[DoF - 1] * s[DoF - 1];
+  for (int c = 0; c < CH; ++c) so[t * CS + c] = acc[c];
+  __syncwarp();
+  const int pairs = (int)min(32LL, total - first - warp);   // (element, level) pairs of this warp
+  double *ow = out + (first + warp) * OP2 + c0;
+  if (OP2 == CH) {
+    for (int y = lane; y < pairs * CH; y += 32) ow[y] = so[warp * CS + (CS == CH ? y : y / CH * CS + y % CH)];
+  } else {
+    for (int y = lane; y < pairs * CH; y += 32) {
+      const int r = y / CH, c = y % CH;
+      if (c < nc) ow[(size_t)r * OP2 + c] = so[(warp + r) * CS + c];
     }
-    out[(size_t)k * per + (size_t)lz * OP2] = acc;
   }
 }
 

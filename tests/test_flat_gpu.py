@@ -139,3 +139,51 @@ def test_output_tiles(oracle_mod, built_lib, cuda_ok, case):
     for k, c in enumerate(codes):
         assert np.array_equal(out[k].reshape(-1), ref[c].reshape(-1, order="F")), (k, c)
     d.close()
+
+
+@pytest.mark.parametrize("OP", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("case", [(2, 4, 9), (2, 3, 17), (12, 2, 33), (2, 1, 64)])
+def test_output_single_quantities(oracle_mod, built_lib, cuda_ok, case, OP):
+    """Every quantity in a call of its own, on grids below and above the size
+    at which a thread takes more sub-cells."""
+    from cgd_b200 import Dycore, _lib, output
+    n, p, nz = case
+    o, g, U, nu = make_case(oracle_mod, n, p, nz, 1, "quadratic")
+    U = _moving(o, U)
+    d = Dycore(g, 1, nu)
+    inter = output.vtk_inter(p, OP, g.xw)
+    f = lambda k: np.asfortranarray(U[..., k])
+    ref = {_lib.OUT_RHO: o.interpolate(f(0), inter), _lib.OUT_PRES: o.interpolate(f(4), inter, kind=1),
+           _lib.OUT_WB: o.interpolate_wb(f(1), f(1), f(3), inter), _lib.OUT_VORT: o.interpolate_vort(U, inter),
+           _lib.OUT_WB_UV: o.interpolate_wb(f(1), f(2), f(3), inter),
+           _lib.OUT_TR: o.interpolate(f(5), inter, rhoc=f(0))}
+    for c, r in ref.items():
+        assert np.array_equal(d.output_fields(U, [c], inter).reshape(-1), r.reshape(-1, order="F")), c
+    # formed quantities on both sides of a launch's sixteen
+    codes = [_lib.OUT_PRES, _lib.OUT_WB] + [_lib.OUT_RHO] * 14 + [_lib.OUT_VORT, _lib.OUT_WB, _lib.OUT_PRES, _lib.OUT_WB_UV]
+    for k, a in enumerate(d.output_fields(U, codes, inter)):
+        assert np.array_equal(a.reshape(-1), ref[codes[k]].reshape(-1, order="F")), (k, codes[k])
+    d.close()
+
+
+@pytest.mark.parametrize("OP", [1, 2, 5])
+def test_output_quotients_at_the_limits(oracle_mod, built_lib, cuda_ok, OP):
+    """c / rho with zeros, infinities, NaN and values whose quotients leave the
+    range of the shared reciprocal; weights of any size."""
+    from cgd_b200 import Dycore, output
+    o, g, U, nu = make_case(oracle_mod, 2, 4, 9, 0, "quadratic")
+    d = Dycore(g, 0, nu)
+    rng = np.random.Generator(np.random.PCG64(17))
+    edge = np.array([0.0, -0.0, 1e-310, 1e-200, 1e-130, 1.0, -3.0, 1e130, 1e200, 1e308, np.inf, np.nan])
+    c = np.asfortranarray(rng.uniform(-2, 2, d.shape[:2]))
+    r = np.asfortranarray(rng.uniform(0.1, 2, d.shape[:2]))
+    at = rng.random(c.shape) < 0.05
+    c[at] = rng.choice(edge, at.sum())
+    at = rng.random(c.shape) < 0.01
+    r[at] = rng.choice(edge, at.sum())
+    for scale in (1.0, 1e-120, 1e120):
+        inter = np.asfortranarray(output.vtk_inter(4, OP, g.xw) * scale)
+        with np.errstate(all="ignore"):
+            ref = o.interpolate(c, inter, rhoc=r)
+        assert np.array_equal(d.interpolate(c, inter, rhoc=r), ref, equal_nan=True), scale
+    d.close()
