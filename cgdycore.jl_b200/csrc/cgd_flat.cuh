@@ -402,7 +402,7 @@ __device__ __forceinline__ void phase2_scalars_flat(const GP &P, const double *_
       DI[k] = (R)P.D[I + N * k];
       DJ[k] = (R)P.D[Jn + N * k];
     }
-    const R rJ = (R)hn[H_RJ * DoF], rhoR = (R)rho;
+    const R rJ = (R)hn[H_RJ * DoF];
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
       const R *c = sc + q * PL + row;
@@ -412,10 +412,10 @@ __device__ __forceinline__ void phase2_scalars_flat(const GP &P, const double *_
         Dx = fsum1(Dx, DI[k], c[k + N * Jn]);
         Dy = fsum1(Dy, DJ[k], c[I + N * k]);
       }
-      const R Gx = (h11 * Dx + h21 * Dy) * rJ * rhoR;
-      const R Gy = (h12 * Dx + h22 * Dy) * rJ * rhoR;
-      s2[(2 * q) * PL + si] = h11 * Gx + h12 * Gy;
-      s2[(2 * q + 1) * PL + si] = h21 * Gx + h22 * Gy;
+      const R Gx = (h11 * Dx + h21 * Dy) * rJ;
+      const R Gy = (h12 * Dx + h22 * Dy) * rJ;
+      s2[(2 * q) * PL + si] = (R)(rho * (h11 * Gx + h12 * Gy));   // (in FP64 in the mixed form too)
+      s2[(2 * q + 1) * PL + si] = (R)(rho * (h21 * Gx + h22 * Gy));
     }
     // D (rho u) at the summed nodes, shared by rho and every scalar
     const R *uc = scon + row, *vc = scon + PL + row;

@@ -69,3 +69,27 @@ def test_mixed_is_deterministic(pair):
     dm.time_stepper(a, 300.0, 3)
     dm.time_stepper(b, 300.0, 3)
     assert np.array_equal(a, b)
+
+
+def test_density_enters_the_hyperviscosity_in_fp64(oracle_mod, built_lib, cuda_ok):
+    """At rest only the hyperviscosity of theta is left, and rho scales its
+    second round.  rho = 1 + 2^-24, which FP32 rounds to 1: the FP64 product
+    rounds every operand up by one unit, 2^-24 to 2^-23 of it; a density rounded
+    first changes nothing."""
+    from cgd_b200 import Dycore
+    o, g, U, nu = make_case(oracle_mod, 6, 4, 20, 0, "uniform")
+    rng = np.random.Generator(np.random.PCG64(23))
+    theta = 300.0 + rng.uniform(-1.0, 1.0, U.shape[:2])
+    eps = 2.0 ** -24
+    for flat in (True, False):
+        d = Dycore(g, 0, nu, precision="mixed")
+        d.set_flat_form(flat)
+        assert d.flat_form() == flat
+        total = []
+        for rho in (1.0, 1.0 + eps):
+            V = np.zeros(U.shape, order="F")
+            V[..., 0] = rho
+            V[..., 4] = rho * theta
+            total.append(np.abs(d.fcn(V)[..., 4]).sum())
+        d.close()
+        assert 0.5 * eps <= total[1] / total[0] - 1.0 <= 3.0 * eps, (flat, total)
