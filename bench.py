@@ -269,11 +269,17 @@ def step_bytes(cfg):
     return tot + 3 * S + 8 * Sp + 5 * NV * S
 
 
-def step_launches(nf, p, nz):
-    """Kernel launches of one captured step of nf elements: phase 1, phase 2
-    and the column kernel in three stages; phase 2 is two launches from 4096
-    CTAs a role on (one per element and 16 levels, 32 at p = 1)."""
-    return 3 * (3 if nf * -(-nz // (32 if p == 1 else 16)) < 4096 else 4)
+def step_launches(ranges, p, nz, nt=0, mixed=False):
+    """Kernel launches of one step whose phases 1 and 2 run over `ranges` elements
+    each (one range of a whole grid; a rank's boundary and interior): phase 1,
+    phase 2 and the column kernel in three stages; phase 2 is two launches from
+    p2_split_threads threads a role on (16 levels a CTA, 32 at p = 1)."""
+    LT = 32 if p == 1 else 16
+    split = (500000 if mixed else 750000) * (2 + nt)
+    n = 1
+    for nf in ranges:
+        n += 2 + (nf * -(-nz // LT) * LT * (p + 1) ** 2 >= split) if nf else 0
+    return 3 * n
 
 
 def ncu_traffic():
@@ -642,7 +648,7 @@ def ensemble_measure(K, warmup, rank, ranks, torch):
             "mass_drift_fp64_max": float(max(abs(x) for x in res["fp64"]["drift"])),
             "finite": res["fp64"]["finite"] and res["mixed"]["finite"],
             "perturbation": f"theta +-{E['theta_amp']} K, u,v +-{E['wind_amp']} m/s, seed {E['seed0']}+member",
-            "gpu_launches": {"fused": 3, "members": sum(step_launches(m[0].NF, 4, m[0].nz) for m in members)}.get(
+            "gpu_launches": {"fused": 3, "members": sum(step_launches([m[0].NF], 4, m[0].nz) for m in members)}.get(
                 res["fp64"]["tuning"].split("stage=")[1].split(";")[0], 9) * K}
 
 
@@ -843,7 +849,7 @@ def run_ours(args, cfg, rank, world, local):
             "adjoint": adjoint,
             "ensemble": ensemble,
             "output": outp,
-            "gpu_launches": step_launches(6 * cfg.nPanel ** 2, cfg.OrdPoly, cfg.nz) * args.steps,
+            "gpu_launches": step_launches([6 * cfg.nPanel ** 2], cfg.OrdPoly, cfg.nz, cfg.NumTr) * args.steps,
             "cpu_baseline": cpu,
             "clocks": clk,
         }
@@ -919,7 +925,7 @@ def run_shard(args, cfg, rank, world, local):
                 "e2e": {"value": Ke / te, "unit": UNIT, "h2d_bytes_per_step": tot_bytes,
                         "d2h_bytes_per_step": tot_bytes, "steps": Ke,
                         "call": "cgd_ros_step(h_rank, host_part, dt, 1) per step on every rank"},
-                "gpu_launches": (step_launches(6 * cfg.nPanel ** 2 // world, cfg.OrdPoly, cfg.nz) + (12 if world > 1 else 0)) * args.steps, "clocks": clk}
+                "gpu_launches": (step_launches([P.nb_boundary, P.NF - P.nb_boundary], cfg.OrdPoly, cfg.nz, cfg.NumTr) + (12 if world > 1 else 0)) * args.steps, "clocks": clk}
         print(json.dumps(line), flush=True)
     d.close()
     if world > 1:

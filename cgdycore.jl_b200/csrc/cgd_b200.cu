@@ -279,7 +279,7 @@ void launch_p2r(cgd_handle *h, const double *U, const double *Pr, const double *
       cudaFuncSetAttribute(k_phase2_scalars<N, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FF::S_BYTES);
     }
     const dim3 half(grid.x / 2, grid.y);
-    if ((long long)half.x * half.y < P2_SPLIT_MIN) {
+    if ((long long)half.x * half.y * FF::THREADS < p2_split_threads<N, NT, R>()) {
       k_phase2_flat<N, NT, R><<<grid, FF::THREADS, FF::SMEM, h->stream>>>(gp, U, Pr, C1, C);
     } else {
       k_phase2_momentum<N, R><<<half, FF::THREADS, FF::M_BYTES, h->stream>>>(gp, U, Pr, C1, C);

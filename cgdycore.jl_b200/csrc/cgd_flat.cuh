@@ -701,14 +701,26 @@ __global__ void __launch_bounds__(P2Flat<N, NT, R>::THREADS, P2Flat<N, NT, R>::M
 
 // The roles in launches of their own: the scalars' needs fewer registers, so
 // that half as many CTAs again fit an SM (48 registers; at p = 4 three CTAs
-// instead of two), which one launch of both cannot use.  From P2_SPLIT_MIN CTAs
-// of each role on (some 14 waves of the momentum role).  One launch -> two, ms:
-// nPanel 60, nz 64 3.37 -> 3.16 (86400 CTAs); nPanel 30, nz 45, two tracers
-// 0.790 -> 0.784 (16200); nPanel 30, p 3, nz 31 0.270 -> 0.261 (10800); below,
-// the second launch's tail and start cost more: nPanel 16, nz 30 0.1305 ->
-// 0.1321 (3072), nPanel 6, nz 10 0.018 -> 0.021 (216).  The momentum role at 48
-// registers spills and takes longer (0.89 for 0.79 together).
-constexpr int P2_SPLIT_MIN = 4096;
+// instead of two), which one launch of both cannot use.  Against it stand the
+// second launch's start and tail.  The crossover lies at as many threads of a
+// role for every p, later with tracers, which take registers and shared memory
+// of the scalars' gain, and earlier in the mixed form.  One launch / two, us:
+//
+//              no tracer                      two tracers
+//   p 4        1.23 M threads 131 / 132       1.92 M threads 244 / 250
+//              1.92 M         201 / 199       4.87 M         599 / 595
+//              17.3 M        1754 / 1641      17.3 M        2140 / 2069
+//   p 4 mixed  1.04 M threads 103 / 101       1.04 M threads 125 / 124
+//   p 2        1.04 M threads 95.2 / 95.9     2.33 M threads 253 / 255
+//              1.75 M         159 / 157       4.15 M         444 / 438
+//   p 1        1.04 M threads 70.3 / 70.7     1.38 M threads 117 / 119
+//              1.38 M         94.2 / 91.5     2.46 M         204 / 202
+//
+// (A line at 4096 CTAs, whatever their size, cost up to 7 % at p 1 and 2.)  The
+// momentum role at 48 registers spills and takes longer (0.89 for 0.79 ms of
+// both, drop-in grid).
+template <int N, int NT, typename R>
+constexpr long long p2_split_threads() { return (sizeof(R) == sizeof(float) ? 500000LL : 750000LL) * (2 + NT); }
 
 template <int N, typename R>
 __global__ void __launch_bounds__(P2Flat<N, 0, R>::THREADS, P2Flat<N, 0, R>::MINB)

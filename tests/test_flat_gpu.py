@@ -187,3 +187,38 @@ def test_output_quotients_at_the_limits(oracle_mod, built_lib, cuda_ok, OP):
             ref = o.interpolate(c, inter, rhoc=r)
         assert np.array_equal(d.interpolate(c, inter, rhoc=r), ref, equal_nan=True), scale
     d.close()
+
+
+@pytest.mark.parametrize("case", [(16, 4, 48, 0, False), (25, 4, 32, 2, False), (21, 4, 48, 4, True), (20, 3, 48, 0, False),
+                                  (25, 3, 48, 1, True), (26, 2, 48, 0, False), (38, 2, 33, 3, True), (33, 1, 33, 0, False),
+                                  (45, 1, 33, 2, True)])
+def test_phase2_launch_forms(built_lib, cuda_ok, case):
+    """From p2_split_threads threads a role on, a handle runs the roles of phase
+    2 in launches of their own, an ensemble always in one: the same bits."""
+    import torch
+    from cgd_b200 import Dycore, Ensemble, physics
+    from cgd_b200 import grid as G
+    n, p, nz, nt, mixed = case
+    role = 6 * n * n * -(-nz // (32 if p == 1 else 16)) * (32 if p == 1 else 16) * (p + 1) ** 2
+    assert role >= (500000 if mixed else 750000) * (2 + nt)
+    g = G.init_grid_sphere_device(n, p, G.vertical_quadratic(nz, 30000.0), 30000.0, 6.371e6)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    U = torch.rand((5 + nt, g.NumG, nz), dtype=torch.float64, device="cuda", generator=gen) * 0.01 + 1.0
+    U[1:4] = 10.0 * (U[1:4] - 1.005)
+    U[4] *= 300.0
+    out = []
+    for ensemble in (False, True):
+        d = Dycore(g, nt, physics.hyperdiffusion(n, p), precision="mixed" if mixed else "fp64")
+        assert d.flat_form()
+        V = U.clone()
+        if ensemble:
+            e = Ensemble([d])
+            e.step([V], [10.0], 1)
+            e.close()
+        else:
+            d.time_stepper(V, 10.0, 1)
+        d.close()
+        out.append(V)
+    assert bool(torch.isfinite(out[0]).all())
+    assert torch.equal(out[0], out[1])
