@@ -65,11 +65,6 @@ __device__ __forceinline__ void cp_async8(double *smem_dst, const double *gsrc)
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
-__device__ __forceinline__ void cp_async4(float *smem_dst, const float *gsrc)
-{
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gsrc) : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // Ask for the bytes at p in L2 (whole 16-byte units, from the one p lies in)
@@ -171,20 +166,6 @@ __device__ __forceinline__ void physics_terms(const GP &P, int l, int g, double 
     f[4] += -rhoth / T * DeltaT;
   }
   if (P.damping) f[3] += -P.dampc[l + (size_t)P.nz * g] * w;
-}
-
-// RecU4: src/GPU/OperatorKernel.jl:1044-1059
-__device__ __forceinline__ void recu4(double cLL, double cL, double cR, double cRR, double JLL,
-                                      double JL, double JR, double JRR, double &cFL, double &cFR)
-{
-  double kR = (JL / (JL + JR)) * ((JLL + JL) / (JLL + JL + JR));
-  double kL = (JL / (JLL + JL)) * (JR / (JLL + JL + JR));
-  double r = (cL - cLL) / (cR - cL + 1.e-20);
-  cFL = cL + cgd_max(0.0, cgd_min(r, cgd_min(kL * r + kR, 1.0))) * (cR - cL);
-  kL = (JR / (JR + JL)) * ((JRR + JR) / (JL + JR + JRR));
-  kR = (JR / (JRR + JR)) * (JL / (JL + JR + JRR));
-  r = (cR - cRR) / (cL - cR + 1.e-20);
-  cFR = cR + cgd_max(0.0, cgd_min(r, cgd_min(kR * r + kL, 1.0))) * (cL - cR);
 }
 
 // ---------------------------------------------------------------------------

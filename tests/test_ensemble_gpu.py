@@ -146,3 +146,33 @@ def test_member_changes_its_layers(oracle_mod, built_lib, cuda_ok, form):
     ens.close()
     for d, _, _ in mem + alone:
         d.close()
+
+
+@pytest.mark.parametrize("form", ["split", "fused", "members", "autotune"])
+def test_flat_and_general_members_together(oracle_mod, built_lib, cuda_ok, form):
+    """One member's metric is off the flat form: the ensemble has work lists of
+    both kinds, and every member comes out as on its own."""
+    import dataclasses
+    from cgd_b200 import Dycore, Ensemble
+    mem, ref = [], []
+    for i, (n, p, nz, st, dt) in enumerate(MEMBERS):
+        o, g, U, nu = make_case(oracle_mod, n, p, nz, 0, st, noise=0.01 + 0.01 * i)
+        if i == 1:
+            dX = np.array(g.dXdxI, order="F")
+            dX[..., 5, -1] *= 1.0 + 1e-3
+            g = dataclasses.replace(g, dXdxI=dX)
+        mem.append((Dycore(g, 0, nu), _dev(U), dt))
+        V = _dev(U)
+        d = Dycore(g, 0, nu)
+        d.time_stepper(V, dt, 2)
+        d.close()
+        ref.append(V)
+    assert [d.flat_form() for d, _, _ in mem] == [True, False, True]
+    ens = Ensemble([d for d, _, _ in mem], autotune=form == "autotune", fused=form == "fused",
+                   members_form=form == "members")
+    ens.step([U for _, U, _ in mem], [dt for _, _, dt in mem], 2)
+    for (_, U, _), V in zip(mem, ref):
+        assert np.array_equal(_host(U), _host(V))
+    ens.close()
+    for d, _, _ in mem:
+        d.close()

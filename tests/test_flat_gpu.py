@@ -41,6 +41,7 @@ def test_flat_tendency_and_step(oracle_mod, built_lib, cuda_ok, case):
     o, g, U, nu = make_case(oracle_mod, n, p, nz, nt, "quadratic")
     U = _moving(o, U)
     d = Dycore(g, nt, nu)
+    assert d.flat_form()
     err = rel_err_per_field(d.fcn(U), o.rhs(U))
     assert (err <= _tol(5 + nt)).all(), err
     V = np.array(U, order="F")
@@ -68,6 +69,7 @@ def test_general_metric(oracle_mod, built_lib, cuda_ok, case):
     Fo = o.rhs(U)
     for exact in (True, False):
         d = Dycore(g, nt, nu, exact=exact)
+        assert not d.flat_form()
         F = d.fcn(U)
         d.close()
         if exact:
@@ -89,6 +91,7 @@ def test_flat_adjoint(oracle_mod, built_lib, cuda_ok, case):
     out = []
     for exact in (True, False):
         d = Dycore(g, 0, nu, exact=exact)
+        assert d.flat_form() != exact
         out.append(d.fcn_adjoint(U, L))
         d.close()
     err = rel_err_per_field(out[1], out[0])
@@ -107,6 +110,7 @@ def test_layers_are_checked(oracle_mod, built_lib, cuda_ok):
     F0 = None
     for layers in (None, z, z * 1.01 ** np.arange(9)):
         d = Dycore(dataclasses.replace(g, layers=layers), 1, nu)
+        assert d.flat_form() == (layers is None or layers is z)
         F = d.fcn(U)
         d.close()
         assert (rel_err_per_field(F, Fo) <= _tol(6)).all()
@@ -222,3 +226,29 @@ def test_phase2_launch_forms(built_lib, cuda_ok, case):
         out.append(V)
     assert bool(torch.isfinite(out[0]).all())
     assert torch.equal(out[0], out[1])
+
+
+def _workload_grids():
+    from cgd_b200 import physics as Ph
+    out = {(c.nPanel, c.OrdPoly, c.nz, c.stretch) for c in Ph.CONFIGS.values()}
+    out |= {(n, Ph.ENSEMBLE["OrdPoly"], nz, "quadratic") for n, nz in Ph.ENSEMBLE["grids"]}
+    return sorted(out | {(12, p, 31, "quadratic") for p in (1, 2, 3)})
+
+
+@pytest.mark.parametrize("where", ["host", "device"])
+@pytest.mark.parametrize("case", _workload_grids())
+def test_workload_grids_are_flat(built_lib, cuda_ok, case, where):
+    """The grids of the package's configurations are of the flat form, formed on
+    the device or on the host: a set-up that moved their rounding past the check
+    (2e-15; uniform levels come near it, and above it at nz 45) would lose the
+    flat kernels silently."""
+    from cgd_b200 import Dycore
+    from cgd_b200 import grid as G
+    n, p, nz, stretch = case
+    if where == "host" and n > 16:
+        pytest.skip("minutes on the host")
+    z = G.vertical_uniform(nz, 30000.0) if stretch == "uniform" else G.vertical_quadratic(nz, 30000.0)
+    init = G.init_grid_sphere if where == "host" else G.init_grid_sphere_device
+    d = Dycore(init(n, p, z, 30000.0, 6.371e6))
+    assert d.flat_form()
+    d.close()

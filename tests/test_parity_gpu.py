@@ -229,3 +229,34 @@ def test_two_layers(oracle_mod, lib_ready, variant):
     _same(kg, ko, d.exact, TOL_RHS)
     _same(vg, vo, d.exact, TOL_RHS)
     d.close()
+
+
+@pytest.mark.parametrize("place", ["apart", "misaligned", "same", "overlapping", "over_state"])
+def test_jac_bands_device_arrays(oracle_mod, built_lib, cuda_ok, place):
+    """cgd_jac_bands into device arrays: written by the kernel where they lie
+    apart and aligned, else copied after it in the order of the arguments; the
+    same values as into host arrays either way."""
+    import torch
+    o, g, U, nu = make_case(oracle_mod, 3, 4, 9, 0, "quadratic")
+    from cgd_b200 import Dycore
+    d = Dycore(g, 0, nu)
+    ref = [np.asarray(a).reshape(-1, order="F") for a in d.jac_bands(d.new_bands(), U)]
+    n, S = ref[0].size, U.size
+    buf = torch.zeros(S + 6 * n + 8, dtype=torch.float64, device="cuda")
+    V = buf[:S]
+    V.copy_(torch.from_numpy(np.ascontiguousarray(U.transpose(2, 1, 0))).cuda().reshape(-1))
+    at = {"apart": [S + k * (n + n % 2) for k in range(4)],
+          "misaligned": [S + 1, S + 1 + n, S + 1 + 2 * n, S + 1 + 3 * n],
+          "same": [S, S, S + n, S + n],
+          "overlapping": [S, S + n // 2, S + 2 * n, S + 3 * n],
+          "over_state": [S - 6, S + n, S + 2 * n, S + 3 * n]}[place]
+    before = V.clone()
+    d.jac_bands([buf[a:a + n] for a in at], V)
+    want = torch.full((buf.numel(),), float("nan"), dtype=torch.float64)
+    want[:S] = before.cpu()
+    for a, r in zip(at, ref):
+        want[a:a + n] = torch.from_numpy(np.ascontiguousarray(r))
+    got = buf.cpu()
+    written = ~torch.isnan(want)
+    assert torch.equal(got[written], want[written])
+    d.close()
