@@ -723,7 +723,7 @@ int flat_factors(cgd_handle *h, const double *zin)
   }
   CK(cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
   k_flat_layers<<<1, 64, 0, h->stream>>>(P, zd, h->zl);
-  k_flat_factors<<<h->NF, 32, 0, h->stream>>>(P, h->hm);
+  k_flat_factors<<<h->NF, 256, 0, h->stream>>>(P, h->hm);
   k_flat_check<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(P, std::fabs(2.0 * h->cfg.Omega), h->flag);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(&bad, h->flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
