@@ -19,12 +19,14 @@
 // come from the neighbouring lanes (shuffles within the LT lanes of a node)
 // and, at the tile's ends, from halo rows that a few threads form beforehand.
 //
-// Bound by the L1/shared pipe (61 % of its peak: 98 M shared-load and 72 M
-// global-load wavefronts a launch) and by the latency of its loads and
-// barriers.  One thread per (node, level) instead of one warp per level with
-// 25 of 32 lanes, two roles at 72 registers (26 warps an SM) instead of one at
-// 128 (16 warps): nPanel 30, p 4, nz 45, two tracers 1.327 -> 1.224 ms, mixed
-// form 1.247 -> 1.166 ms, nPanel 60, nz 64 5.65 -> 4.69 ms.
+// Bound by the L1/shared pipe and by the latency of its loads and barriers (61 %
+// of the pipe's peak, 98 M shared-load and 72 M global-load wavefronts a launch,
+// before it summed the phase-1 contributions itself).  One thread per (node,
+// level) instead of one warp per level with 25 of 32 lanes, two roles at 72
+// registers (26 warps an SM) instead of one at 128 (16 warps): nPanel 30, p 4, nz
+// 45, two tracers 1.327 -> 1.224 ms, mixed form 1.247 -> 1.166 ms, nPanel 60, nz 64
+// 5.65 -> 4.69 ms; with the phase-1 sums, which a kernel of 0.11 ms formed before,
+// 1.226, 1.137 and 5.01 ms.
 //
 // The vertical momentum equation lives on interfaces: the contribution of
 // the element node to w at interface l is hi(l) + lo(l+1), hi from the upper

@@ -391,8 +391,7 @@ int cgd_jac_schur_solve_noalloc(const cgd_config *cfg, const double *U, const do
  * CGD_ERR_UNSUPPORTED otherwise), three persistent cooperative launches, one
  * per stage, each running pressure, both tendency phases with their DSS and
  * the column solve and update with a grid barrier between them (fused form;
- * it allocates a second contribution buffer and a second stage state per
- * member; a barrier wait that exceeds a few seconds ends the launch and the
+ * it allocates a second stage state per member; a barrier wait that exceeds a few seconds ends the launch and the
  * step returns CGD_ERR_TIMEOUT).  Calls on different batches must not run
  * concurrently: they share those constant tables.  The member handles must
  * stay alive and must not be stepped on their own while their batch steps.

@@ -1,6 +1,6 @@
 """Batched ensemble on the GPU: members on different grids (nPanel, nz) and
 with different dt advance together through cgd_batch_step, one graph per
-ensemble step: 15 launches (split form), one persistent cooperative launch
+ensemble step: 9 launches (split form), one persistent cooperative launch
 per stage (fused form), or one graph branch per member running that
 member's own step (members form).  All forms run the single-member kernel
 bodies on the same data in the same order, so every member must come out
