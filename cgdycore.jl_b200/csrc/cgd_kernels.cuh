@@ -859,8 +859,9 @@ __device__ __forceinline__ void column_body(const GP &P, const ColArgs &A, const
       if (MODE == 0) {
         // dPresdRhoTh once per level, shared with the interface below
 #ifdef CGD_FAST
-        // Rd (Rd rhotheta / p0)^(kappa/(1-kappa)) = p / rhotheta with the pressure at hand
-        tmp[l] = A.ps[o0] / A.Vn[o0 + 4 * fs];
+        // Rd (Rd rhotheta / p0)^(kappa/(1-kappa)) = p / rhotheta with the pressure at hand (0 at 0)
+        const double rth = A.Vn[o0 + 4 * fs];
+        tmp[l] = rth != 0.0 ? A.ps[o0] / rth : 0.0;
         tmp[LS + l] = 1.0 / P.dz[o0];
 #else
         tmp[l] = dpdrhoth(P, A.Vn[o0 + 4 * fs]);

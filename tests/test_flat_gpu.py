@@ -252,3 +252,17 @@ def test_workload_grids_are_flat(built_lib, cuda_ok, case, where):
     d = Dycore(init(n, p, z, 30000.0, 6.371e6))
     assert d.flat_form()
     d.close()
+
+
+def test_step_where_rho_theta_is_zero(oracle_mod, built_lib, cuda_ok):
+    """dp/d(rho theta) there is 0, as the power gives it, not 0 / 0."""
+    from cgd_b200 import Dycore
+    o, g, U, nu = make_case(oracle_mod, 3, 4, 9, 1, "quadratic")
+    U = _moving(o, U)
+    U[3, 10, 4] = U[0, 50, 4] = U[8, 70, 4] = 0.0
+    d = Dycore(g, 1, nu)
+    V = np.array(U, order="F")
+    d.time_stepper(V, 1e-3, 1)
+    d.close()
+    assert np.isfinite(V).all()
+    assert (rel_err_per_field(V, o.ros_step(U, 1e-3, 1)) <= 1e-9).all()
