@@ -375,14 +375,15 @@ void column(cgd_handle *h, const ColArgs &a)
 }
 
 // The output launches of n quantities, with up to 25 of a quantity's sub-cells a
-// thread.  A launch of few CTAs is bound by a thread's chain of sums and by the
-// second launch itself: below CELLS_SMALL CTAs a thread takes 4 (9 of an odd
-// OrdPrint) and k_cells starts while k_cells_nodal ends.  Above, its waiting CTAs
-// would keep that kernel's out: nPanel 60, p 1, nz 40, vorticity 97 -> 107 us.
+// thread.  A launch of few CTAs is bound by a thread's chain of sums: below
+// CELLS_SMALL CTAs a thread takes 4 (9 of an odd OrdPrint; nPanel 6, nz 10,
+// OrdPrint 4, rho 35 -> 31 us).  k_cells starts while k_cells_nodal ends: 3 to 5 us
+// of every call that forms something (nPanel 30, nz 45, w 59 -> 56 us, nine
+// quantities 313 -> 309; nPanel 60, p 1, the vorticity 96 -> 93).
 constexpr unsigned CELLS_SMALL = 2 * 148;
 
 template <int N, int CH>
-void launch_cells_c(cgd_handle *h, const CellArgs &a, int n, int OP, double *cell, bool overlap)
+void launch_cells_c(cgd_handle *h, const CellArgs &a, int n, int OP, double *cell, bool nodal)
 {
   const long long total = (long long)h->nz * h->NF;
   const unsigned groups = (OP * OP + CH - 1) / CH;
@@ -394,7 +395,7 @@ void launch_cells_c(cgd_handle *h, const CellArgs &a, int n, int OP, double *cel
   cfg.blockDim = dim3(CELL_THREADS);
   cfg.stream = h->stream;
   cfg.attrs = at;
-  cfg.numAttrs = overlap ? 1 : 0;
+  cfg.numAttrs = nodal ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k_cells<N, CH>, (const GP)h->gp, (const CellArgs)a, (const double *)h->ointer, OP * OP, cell);
 }
 
@@ -408,18 +409,16 @@ void launch_cells_n(cgd_handle *h, NodalArgs na, const CellArgs &a, int n, int O
   const unsigned tiles = na.rot ? (unsigned)((h->nz + CF::LT - 1) / CF::LT) * (unsigned)h->NF : 0;
   const unsigned nodal = na.colblocks + na.w0blocks + tiles;
   const bool small = (unsigned)(((long long)h->nz * h->NF + CELL_THREADS - 1) / CELL_THREADS) * n < CELLS_SMALL;
-  const bool overlap = small && nodal;
-  na.overlap = overlap;
   if (nodal > tiles) k_cells_nodal<N, true><<<nodal, CF::THREADS, 0, h->stream>>>(h->gp, na);
   else if (nodal) k_cells_nodal<N, false><<<nodal, CF::THREADS, 0, h->stream>>>(h->gp, na);
   const int CH = OP == 1 ? 1 : small ? (OP % 2 ? 9 : 4) : OP == 6 ? 18 : OP == 8 ? 16 : std::min(OP * OP, 25);
   switch (CH) {
-    case 1: launch_cells_c<N, 1>(h, a, n, OP, cell, overlap); break;
-    case 4: launch_cells_c<N, 4>(h, a, n, OP, cell, overlap); break;
-    case 9: launch_cells_c<N, 9>(h, a, n, OP, cell, overlap); break;
-    case 16: launch_cells_c<N, 16>(h, a, n, OP, cell, overlap); break;
-    case 18: launch_cells_c<N, 18>(h, a, n, OP, cell, overlap); break;
-    default: launch_cells_c<N, 25>(h, a, n, OP, cell, overlap); break;   // OrdPrint 7: 25 + 24
+    case 1: launch_cells_c<N, 1>(h, a, n, OP, cell, nodal > 0); break;
+    case 4: launch_cells_c<N, 4>(h, a, n, OP, cell, nodal > 0); break;
+    case 9: launch_cells_c<N, 9>(h, a, n, OP, cell, nodal > 0); break;
+    case 16: launch_cells_c<N, 16>(h, a, n, OP, cell, nodal > 0); break;
+    case 18: launch_cells_c<N, 18>(h, a, n, OP, cell, nodal > 0); break;
+    default: launch_cells_c<N, 25>(h, a, n, OP, cell, nodal > 0); break;   // OrdPrint 7: 25 + 24
   }
 }
 

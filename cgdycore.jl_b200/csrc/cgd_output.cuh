@@ -37,9 +37,9 @@
 //   vorticity alone    311 -> 145        327 -> 161
 //
 // and nPanel 60, nz 64, seven quantities, OrdPrint 1 2718 -> 1260; nPanel 6, nz 10
-// 37 -> 36 (of these some 25 us are the call's own).  k_cells_nodal reads 0.26 GB
-// of metric at 4.0 TB/s (nPanel 20: 87 us under a profiler), k_cells moves 3.1
-// TB/s (50 us) and waits for its gathers.
+// 37 -> 36 (of these some 25 us are the call's own).  k_cells_nodal moves
+// 4.0 TB/s, most of it the vorticity's metric (nPanel 20: 87 us under a profiler),
+// k_cells 3.1 TB/s (50 us), waiting for its gathers.
 #pragma once
 #include "cgd_kernels.cuh"
 
@@ -71,16 +71,17 @@ struct NodalArgs {
   const double *rho, *rhoth, *u, *v;
   double *p, *th, *w0[2], *rot;
   unsigned colblocks, w0blocks;
-  bool overlap;   // k_cells may start now
 };
 
-template <int N, bool COLS>   // COLS: more than the vorticity
+// COLS: more than the vorticity (without the others' code it alone takes 97 instead
+// of 110 us on nPanel 60, p 1, nz 40)
+template <int N, bool COLS>
 __global__ void __launch_bounds__(NodalCfg<N>::THREADS) k_cells_nodal(const GP P, const NodalArgs A)
 {
   using CF = NodalCfg<N>;
   constexpr int DoF = CF::DoF, LT = CF::LT, RS = CF::RS;
   const int nz = P.nz, t = threadIdx.x;
-  if (A.overlap) asm volatile("griddepcontrol.launch_dependents;\n");   // k_cells waits for this grid's end itself
+  asm volatile("griddepcontrol.launch_dependents;\n");   // k_cells waits for this grid's end itself
   if (COLS && blockIdx.x < A.colblocks) {
     const size_t i = (size_t)blockIdx.x * CF::THREADS + t;
     if (i >= (size_t)nz * P.NumG) return;
